@@ -23,12 +23,14 @@
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
+#include <map>
 #include <mutex>
 #include <string>
 #include <type_traits>
 #include <unordered_map>
 
 #include "dr_device.h"
+#include "dr_gs.cuh"
 #include "dr_kernels.cuh"
 
 namespace dr {
@@ -87,15 +89,6 @@ void cuda_check(cudaError_t e, const char* what, const char* file, int line) {
 
 namespace {
 
-// Lanes per row for the Gauss-Seidel colour kernel: about the mean row length.
-int pick_G(long long nnz, int n) {
-  if (n <= 0) return 1;
-  double avg = (double)nnz / (double)n;
-  int G = 1;
-  while (G < 32 && G < avg * 0.75) G *= 2;
-  return G;
-}
-
 // Greedy packing of consecutive rows into tiles of at most max_rows rows,
 // kTileCap nonzeros and a column span below 65536 (so that a tile's columns
 // are 16-bit offsets from its smallest column).  A row longer than kTileCap,
@@ -152,19 +145,69 @@ static_assert(kTileCap == kRowTileCap, "host and device tile capacities differ")
 // read nothing but sparsity patterns before pdl_wait() (k_tile_rows,
 // k_coarse_tail, k_pcg_update).
 template <typename... KArgs, typename... Args>
-void launch_dependent(void (*kern)(KArgs...), int grid, int block, size_t smem, cudaStream_t st,
-                      Args&&... args) {
+void launch_cluster(int cluster, void (*kern)(KArgs...), int grid, int block, size_t smem, cudaStream_t st,
+                    Args&&... args) {
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = dim3((unsigned)grid);
   cfg.blockDim = dim3((unsigned)block);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = st;
-  cudaLaunchAttribute at[1];
+  cudaLaunchAttribute at[2];
   at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   at[0].val.programmaticStreamSerializationAllowed = 1;
+  at[1].id = cudaLaunchAttributeClusterDimension;
+  at[1].val.clusterDim.x = (unsigned)cluster;
+  at[1].val.clusterDim.y = at[1].val.clusterDim.z = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = cluster > 1 ? 2 : 1;
+  DR_CK(cudaLaunchKernelEx(&cfg, kern, std::forward<Args>(args)...));
+}
+template <typename... KArgs, typename... Args>
+void launch_dependent(void (*kern)(KArgs...), int grid, int block, size_t smem, cudaStream_t st,
+                      Args&&... args) {
+  launch_cluster(1, kern, grid, block, smem, st, std::forward<Args>(args)...);
+}
+
+// Blocks of a one-cluster kernel (16 where the device can place such a
+// cluster, else the portable 8) and its largest dynamic shared memory; the
+// function's limits are raised once per device.
+struct ClusterLimits {
+  int blocks = 0;
+  size_t smem = 0;
+};
+template <typename... KArgs>
+ClusterLimits cluster_limits(void (*kern)(KArgs...), int block) {
+  static std::mutex mu;
+  static std::map<std::pair<const void*, int>, ClusterLimits> cache;
+  int dev = 0;
+  DR_CK(cudaGetDevice(&dev));
+  std::lock_guard<std::mutex> lk(mu);
+  ClusterLimits& c = cache[{(const void*)kern, dev}];
+  if (c.blocks) return c;
+  int optin = 0;
+  cudaFuncAttributes fa{};
+  DR_CK(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
+  DR_CK(cudaFuncGetAttributes(&fa, kern));
+  c.smem = (size_t)optin - fa.sharedSizeBytes;
+  DR_CK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)c.smem));
+  DR_CK(cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(16);
+  cfg.blockDim = dim3((unsigned)block);
+  cfg.dynamicSmemBytes = c.smem;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = 16;
+  at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
   cfg.attrs = at;
   cfg.numAttrs = 1;
-  DR_CK(cudaLaunchKernelEx(&cfg, kern, std::forward<Args>(args)...));
+  int fit = 0;
+  if (cudaOccupancyMaxActiveClusters(&fit, kern, &cfg) != cudaSuccess) {
+    cudaGetLastError();
+    fit = 0;
+  }
+  c.blocks = fit >= 1 ? 16 : 8;
+  return c;
 }
 
 // Blocks of `nt` threads with `smem` dynamic shared memory that fit on one
@@ -318,8 +361,15 @@ DevHier::DevHier(const HostHierarchy& H, int device, const BatchLayout* batch) {
       d.ncolors = h.num_colors;
       d.color_off = h.color_off;
       if (h.num_colors > 0) {
-        d.color_order = alloc<int>(h.color_order.size());
-        h2d(d.color_order, h.color_order, st_);
+        std::vector<int4> meta(h.color_order.size());
+        for (size_t k = 0; k < meta.size(); ++k) {
+          const int i = h.color_order[k];
+          meta[k] = make_int4(i, h.A.rp[i], h.A.rp[i + 1], h.colors[i] - 1);
+        }
+        d.gs_meta = alloc<int4>(meta.size());
+        d.color_offd = alloc<int>(h.color_off.size());
+        DR_CK(cudaMemcpy(d.gs_meta, meta.data(), meta.size() * sizeof(int4), cudaMemcpyHostToDevice));
+        DR_CK(cudaMemcpy(d.color_offd, h.color_off.data(), h.color_off.size() * sizeof(int), cudaMemcpyHostToDevice));
       }
       d.has_rap = h.has_rap_map;
       if (d.has_rap || !h.ap_rp.empty()) up_csr(d.AP, h.A.n, h.P.nc, h.ap_rp, h.ap_ci, nullptr);
@@ -481,7 +531,6 @@ void DevHier::upload_csr(DevMat& M, int n, int m, const std::vector<int>& rp, co
   h2d(M.ci, ci, st_);
   M.v = alloc<double>(ci.size() + 4);
   if (v) h2d(M.v, *v, st_);
-  M.Ggs = pick_G(M.nnz, n);
   M.form = row_form(rp);
   M.maxlen = 0;
   for (int i = 0; i < n; ++i) M.maxlen = std::max(M.maxlen, rp[i + 1] - rp[i]);
@@ -596,6 +645,9 @@ void DevHier::ensure_fp32() {
   fp32_ = true;
   if (at_built_) alloc_transpose_fp32();
   refresh_fp32();
+  // the copies are complete before any kernel that prefetches values ahead
+  // of its wait for the previous kernel (k_gs_color, k_gs_cluster)
+  DR_CK(cudaStreamSynchronize(st_));
   if (!batch_) build_tail();
 }
 
@@ -921,6 +973,45 @@ void DevHier::refresh_fp32() {
 }
 
 // ------------------------------------------------------------ cycle pieces
+// `steps` coloured Gauss-Seidel sweeps on level L, in place: one launch of
+// one cluster when the iterate fits in a block's shared memory and a colour
+// holds, on average, no more rows than the cluster has row groups (one round
+// each; 256 groups of 32 lanes, 1024 of 8); else one launch per colour.  With
+// two rounds a colour the cluster's 16 SMs cannot stream the rows as fast as
+// the whole GPU: level 2 of the 64^3 heterogeneous problem (57 colours of 490
+// rows) takes 173 us per sweep in the cluster and 125 us in 57 launches,
+// level 3 (108 colours of 94 rows) 93 against 280 us.
+template <typename T>
+void DevHier::gs_sweeps(const DevLevel& L, const DevMat& A, const T* b, T* x, int steps) {
+  if (steps <= 0 || A.n <= 0) return;
+  auto run = [&](auto tag) {
+    constexpr int G = decltype(tag)::value;
+    auto kc = k_gs_cluster<G, T>;
+    const ClusterLimits lim = cluster_limits(kc, kern::kGsThreads);
+    const long long groups = (long long)lim.blocks * (kern::kGsThreads / G);
+    const size_t smem = gs_cluster_smem<T>(A.n, (long long)L.ncolors * steps);
+    if (smem <= lim.smem && A.n <= groups * L.ncolors) {
+      counted();
+      launch_cluster(lim.blocks, kc, lim.blocks, kern::kGsThreads, smem, st_, A.n, L.ncolors,
+                     (const int*)L.color_offd, (const int4*)L.gs_meta, (const int*)A.ci, mval<T>(A), b, invd<T>(L),
+                     x, steps, 0, err_flag());
+      return;
+    }
+    for (int s = 0; s < steps; ++s)
+      for (int c = 0; c < L.ncolors; ++c) {
+        const int off = L.color_off[c];
+        const int cnt = L.color_off[c + 1] - off;
+        if (cnt == 0) continue;
+        const int grid = (int)std::min<long long>(((long long)cnt * G + kBlock - 1) / kBlock, max_grid_);
+        counted();
+        launch_dependent(k_gs_color<G, T>, grid, kBlock, 0, st_, cnt, (const int4*)(L.gs_meta + off),
+                         (const int*)A.ci, mval<T>(A), b, invd<T>(L), x);
+      }
+  };
+  if (A.nnz >= 24LL * A.n) run(std::integral_constant<int, 32>{});
+  else run(std::integral_constant<int, 8>{});
+}
+
 template <typename T>
 T* DevHier::smooth(int l, T* x, const T* b, int steps, T* ext, const double* rz_w, bool rz_first) {
   DevLevel& L = L_[l];
@@ -997,24 +1088,7 @@ T* DevHier::smooth(int l, T* x, const T* b, int steps, T* ext, const double* rz_
         x = dst;
       }
   } else {
-    for (int s = 0; s < steps; ++s)
-      for (int c = 0; c < L.ncolors; ++c) {
-        const int off = L.color_off[c];
-        const int cnt = L.color_off[c + 1] - off;
-        if (cnt == 0) continue;
-        const int grid = (int)std::max<long long>(1, std::min<long long>(((long long)cnt * A.Ggs + kBlock - 1) / kBlock, max_grid_));
-        counted();
-        switch (A.Ggs) {
-#define DR_CASE(g)                                                                                  \
-  case g:                                                                                           \
-    k_gs_color<g, T><<<grid, kBlock, 0, st_>>>(cnt, L.color_order + off, A.rp, A.ci, mval<T>(A), b, \
-                                               invd<T>(L), x);                                      \
-    break;
-          DR_CASE(1) DR_CASE(2) DR_CASE(4) DR_CASE(8) DR_CASE(16) DR_CASE(32)
-#undef DR_CASE
-        }
-        DR_CK(cudaGetLastError());
-      }
+    gs_sweeps<T>(L, A, b, x, steps);
   }
   return x;
 }

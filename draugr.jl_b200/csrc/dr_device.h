@@ -101,7 +101,6 @@ struct DevMat {
   double* v = nullptr;
   float* v32 = nullptr;
   RowForm form;       // form of the row kernel
-  int Ggs = 8;        // lanes per row of the Gauss-Seidel colour kernel
   int ntiles = 0;     // row tiles (see k_tile_rows)
   int* tp = nullptr;  // tile row starts, ntiles+1
   int* ts = nullptr;  // tile nonzero starts, ntiles+1
@@ -138,7 +137,8 @@ struct DevLevel {
   float* invd32 = nullptr;
   int ncolors = 0;
   std::vector<int> color_off;  // host copy, num_colors+1
-  int* color_order = nullptr;
+  int* color_offd = nullptr;   // device copy
+  int4* gs_meta = nullptr;     // rows by colour: row, first and last + 1 entry
   bool has_rap = false;
   DevMat AP;                 // pattern and values of A·P (partial resetup)
   SpgemmList ap_list, rap_list;  // product lists of A·P and Pᵀ·(AP), built on the first resetup
@@ -335,6 +335,8 @@ class DevHier {
   template <typename T>
   T* smooth(int l, T* x, const T* b, int steps, T* ext_partner, const double* rz_w = nullptr,
             bool rz_first = false);
+  template <typename T>
+  void gs_sweeps(const DevLevel& L, const DevMat& A, const T* b, T* x, int steps);
   bool fused_rz_ok(const CycleOpts& o) const;
   template <typename T>
   void residual(int l, const T* x, const T* b, T* r, double* rr_dst);

@@ -755,36 +755,6 @@ k_tile_rows(int ntiles, const int* __restrict__ tp, const int* __restrict__ ts,
   if constexpr (DOT) grid_sum_finalize(dacc, partials, ticket, fin);
 }
 
-// Gauss-Seidel update of one colour: rows taken from `order`.
-// x_i += invd_i·(b_i - A_i x)                 (src/smoothers.jl:203-217)
-template <int G, typename T>
-__global__ void __launch_bounds__(kBlock)
-k_gs_color(int cnt, const int* __restrict__ order, const int* __restrict__ rp,
-           const int* __restrict__ ci, const T* __restrict__ av, const T* __restrict__ b,
-           const T* __restrict__ invd, T* x) {
-  constexpr int RPW = 32 / G;
-  const int lane = threadIdx.x & (G - 1);
-  const int g = (threadIdx.x & 31) / G;
-  const long long warp = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const long long nwarps = ((long long)gridDim.x * blockDim.x) >> 5;
-  for (long long base = warp * RPW; base < cnt; base += nwarps * RPW) {
-    const int idx = (int)(base + g);
-    const bool valid = idx < cnt;
-    int row = 0, s = 0, e = 0;
-    if (valid) {
-      row = __ldg(order + idx);
-      s = __ldg(rp + row);
-      e = __ldg(rp + row + 1);
-    }
-    T sum = T(0);
-    // x of the same colour is never a neighbour, so plain loads are safe
-    for (int k = s + lane; k < e; k += G) sum += __ldg(av + k) * x[__ldg(ci + k)];
-#pragma unroll
-    for (int off = G >> 1; off > 0; off >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, off);
-    if (valid && lane == 0) x[row] += __ldg(invd + row) * (__ldg(b + row) - sum);
-  }
-}
-
 // ------------------------------------------------------------ vector kernels
 template <typename T>
 __global__ void k_scale_jacobi_zero(int n, const T* __restrict__ b, const T* __restrict__ invd,

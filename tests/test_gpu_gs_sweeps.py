@@ -1,0 +1,74 @@
+"""Coloured Gauss-Seidel sweeps against NumPy at the sizes where their kernels
+change: rows longer than a group's registers hold, colours larger than the
+cluster's row groups, the largest iterate that fits in shared memory and the
+first that does not, short and long rows, one and several sweeps."""
+
+import numpy as np
+import pytest
+import scipy.sparse as sp
+
+import draugr
+from draugr import problems
+
+pytestmark = pytest.mark.gpu
+
+
+def long_rows(n, nlong, length):
+    rng = np.random.default_rng(5)
+    A = problems.poisson1d(n).tolil()
+    for i in range(nlong):
+        cols = rng.choice(n, size=length, replace=False)
+        A[i, cols] = -0.01
+        A[cols, i] = -0.01
+        A[i, i] = 4.0 + 0.02 * length
+    A = sp.csr_matrix(A)
+    A.sort_indices()
+    return A
+
+
+def banded(n, width):
+    """Every row coupled to the next `width` ones: width + 1 colours."""
+    offs = range(-width, width + 1)
+    return sp.diags([np.full(n - abs(o), 2.0 * width if o == 0 else -1.0) for o in offs], list(offs),
+                    format="csr").sorted_indices()
+
+
+def sweeps(A, order, off, invd, x, b, steps):
+    x = x.copy()
+    for _ in range(steps):
+        for c in range(len(off) - 1):
+            rows = order[off[c]:off[c + 1]]
+            x[rows] += invd[rows] * (b[rows] - A[rows] @ x)
+    return x
+
+
+CASES = {
+    "rows_700_short": lambda: long_rows(3000, 3, 700),          # 8 lanes per row, remainder loop
+    "rows_900_long": lambda: long_rows(400, 40, 390),           # 32 lanes per row
+    "poisson1d_5": lambda: problems.poisson1d(5),
+    "poisson2d_46": lambda: problems.poisson2d(46, 44),         # 2 colours of 1012 rows: the cluster
+    "poisson2d_47": lambda: problems.poisson2d(47, 46),         # of 1081: a launch per colour
+    "fe27_15": lambda: problems.anisotropic_27pt(15),           # 8 colours of about 420 rows: a launch per colour
+    "banded_27000": lambda: banded(27000, 115),                 # 116 colours: FP64 iterate just fits
+    "banded_29100": lambda: banded(29100, 115),                 # it does not
+}
+
+
+@pytest.mark.parametrize("smoother", [draugr.ColoredGaussSeidelType, draugr.L1ColoredGaussSeidelType])
+@pytest.mark.parametrize("name", list(CASES))
+def test_gs_sweeps(name, smoother):
+    A = CASES[name]()
+    n = A.shape[0]
+    h = draugr.amg_setup(A, draugr.AMGConfig(coarsening=draugr.AggregationCoarsening(0.25), smoother=smoother(),
+                                             max_coarse_size=2, max_levels=3))
+    order, off, invd = h.export(0, "color_order"), h.export(0, "color_offsets"), h.export(0, "invdiag")
+    rng = np.random.default_rng(1)
+    x, b = rng.uniform(-1, 1, n), rng.uniform(-1, 1, n)
+    longest = int(np.diff(A.indptr).max())
+    for steps in (1, 2, 3):
+        ref = sweeps(A, order, off, invd, x, b, steps)
+        for prec, eps in ((0, 2.2e-16), (1, 1.2e-7)):
+            got = h.level_op(0, 2, x, b, steps=steps, precision=prec)
+            # a row's sum of `longest` products in another order, every sweep
+            tol = 4 * eps * longest * steps
+            assert np.linalg.norm(got - ref) <= tol * np.linalg.norm(ref), (steps, prec)
