@@ -456,7 +456,7 @@ DevHier::DevHier(const HostHierarchy& H, int device, const BatchLayout* batch) {
           // anyway: apply each coarsest system's explicit inverse
           if (!binv_) binv_ = alloc<double>(std::max<size_t>(batch->lu.size(), 1));
           counted();
-          k_lu_inverse_batch<<<b.nblk, kern::kInvMax, 0, st_>>>(b.nb, b.luoff, b.poff, blu_, bpiv_, binv_);
+          k_lu_inverse_batch<<<b.nblk, kern::kInvThreads, 0, st_>>>(b.nb, b.luoff, b.poff, blu_, bpiv_, binv_);
           DR_CK(cudaGetLastError());
           b.inv = true;
         }
@@ -761,7 +761,7 @@ void DevHier::build_tail() {
     tail_ = l;
   }
   if (tail_ >= nl) return;
-  tail_inv_ = cinv_ok_ && nc_ <= 32;
+  tail_inv_ = cinv_ok_;
   const int cnt = nl - tail_;
   std::reverse(ords.begin(), ords.end());  // tail_ first
   std::vector<int*> ord_dev(cnt);
@@ -933,7 +933,7 @@ void DevHier::build_q(DevLevel& d) {
 void DevHier::build_cinv() {
   if (!cinv_) cinv_ = alloc<double>((size_t)nc_ * nc_);
   counted();
-  k_lu_inverse<<<1, kern::kInvMax, 0, st_>>>(nc_, clu_, cpiv_, cinv_);
+  k_lu_inverse<<<1, kern::kInvThreads, 0, st_>>>(nc_, clu_, cpiv_, cinv_);
   DR_CK(cudaGetLastError());
 }
 
@@ -1104,7 +1104,7 @@ void DevHier::residual(int l, const T* x, const T* b, T* r, double* rr_dst) {
 }
 
 template <typename T>
-void DevHier::coarse_solve(const T* b, T* x) {
+void DevHier::coarse_solve(const T* b, T* x, bool inverse_allowed) {
   int threads = 32;
   while (threads < nc_ && threads < 1024) threads *= 2;
   // stage the factors in shared memory when they fit in 40 KB (n_c <= 70)
@@ -1115,6 +1115,10 @@ void DevHier::coarse_solve(const T* b, T* x) {
   if (tr_) {  // A_c^T y = b with the factors of A_c (adjoint solves)
     k_lu_solve_t<T><<<1, 32, ybytes, st_>>>(nc_, clu_, cpiv_, b, x);
     DR_CK(cudaGetLastError());
+    return;
+  }
+  if (cinv_ok_ && inverse_allowed) {
+    launch_dependent(k_inv_apply<T>, 1, kern::kInvMax, 0, st_, nc_, (const double*)cinv_, b, x);
     return;
   }
   k_lu_solve<T><<<1, threads, ybytes + (staged ? lbytes : 0), st_>>>(nc_, clu_, cpiv_, b, x, staged);
@@ -1199,7 +1203,7 @@ T* DevHier::cycle_level(int l, T* x, const T* b, bool x_zero, const CycleOpts& o
   } else {
     xn = coarse_x<T>();
     if (batch_) batch_coarse<T>(l + 1, bn, xn);
-    else coarse_solve<T>(bn, xn);
+    else coarse_solve<T>(bn, xn, true);
   }
   if (L.fuse_up && !tr_ && o.post >= 1 && !rz_w) {
     // correction and the first post-smoothing step in one pass over Q
@@ -1322,6 +1326,13 @@ void DevHier::build_transpose() {
   DR_CK(cudaStreamSynchronize(st_));
 }
 
+void DevHier::l1_invdiag(const DevMat& M, double* invd) {
+  if (M.n >= 65536)
+    k_l1_invdiag<16><<<grid1d(2LL * M.n, max_grid_), kBlock, 0, st_>>>(M.n, M.rp, M.v, invd);
+  else
+    k_l1_invdiag<4><<<grid1d(8LL * M.n, max_grid_), kBlock, 0, st_>>>(M.n, M.rp, M.v, invd);
+}
+
 void DevHier::refresh_transpose() {
   for (auto& d : L_) {
     if (d.A.nnz > 0) {
@@ -1330,7 +1341,7 @@ void DevHier::refresh_transpose() {
     }
     counted();
     if (d.smoother == SmootherKind::L1Jacobi)
-      k_l1_invdiag<<<grid1d(d.A.n, max_grid_), kBlock, 0, st_>>>(d.A.n, d.At.rp, d.At.v, d.invdT);
+      l1_invdiag(d.At, d.invdT);
     else if (d.smoother == SmootherKind::SPAI0)
       k_spai0_diag<<<grid1d(d.A.n, max_grid_), kBlock, 0, st_>>>(d.A.n, d.At.rp, d.At.ci, d.At.v, d.invdT);
     else
@@ -2165,7 +2176,7 @@ void DevHier::resetup_values(const double* v_dev) {
     counted();
     if (d.smoother == SmootherKind::L1Jacobi || d.smoother == SmootherKind::L1ColoredGS ||
         d.smoother == SmootherKind::L1SerialGS)
-      k_l1_invdiag<<<grid1d(d.A.n, max_grid_), kBlock, 0, st_>>>(d.A.n, d.A.rp, d.A.v, d.invd);
+      l1_invdiag(d.A, d.invd);
     else if (d.smoother == SmootherKind::SerialGS)
       k_sgs_invdiag<<<grid1d(d.A.n, max_grid_), kBlock, 0, st_>>>(d.A.n, d.A.rp, d.A.ci, d.A.v, d.invd);
     else if (d.smoother == SmootherKind::SPAI0)
@@ -2265,10 +2276,14 @@ void DevHier::resetup_values(const double* v_dev) {
   counted();
   k_csr_to_dense<<<grid1d(nc_, max_grid_), kBlock, 0, st_>>>(nc_, C_.rp, C_.ci, C_.v, cdense_);
   DR_CK(cudaMemcpyAsync(clu_, cdense_, (size_t)nc_ * nc_ * sizeof(double), cudaMemcpyDeviceToDevice, st_));
-  int threads = 32;
-  while (threads < nc_ && threads < 1024) threads *= 2;
   counted();
-  k_lu_factor<<<1, threads, 0, st_>>>(nc_, clu_, cpiv_, info_);
+  if (nc_ <= kern::kInvMax) {
+    k_lu_factor_small<<<1, kern::kLuThreads, 0, st_>>>(nc_, clu_, cpiv_, info_);
+  } else {
+    int threads = 32;
+    while (threads < nc_ && threads < 1024) threads *= 2;
+    k_lu_factor<<<1, threads, 0, st_>>>(nc_, clu_, cpiv_, info_);
+  }
   DR_CK(cudaGetLastError());
   if (cinv_ok_) build_cinv();
   if (at_built_) refresh_transpose();  // before the FP32 copies, which include the transposed ones

@@ -341,7 +341,7 @@ class DevHier {
   template <typename T>
   void residual(int l, const T* x, const T* b, T* r, double* rr_dst);
   template <typename T>
-  void coarse_solve(const T* b, T* x);
+  void coarse_solve(const T* b, T* x, bool inverse_allowed = false);
 
   void ensure_fp32();
   void refresh_fp32();
@@ -390,6 +390,7 @@ class DevHier {
   bool tr_ = false;          // cycle pieces use A^T (and the transposed coarsest solve)
   void build_transpose();
   void refresh_transpose();
+  void l1_invdiag(const DevMat& M, double* invd);
   double* bk_[8] = {nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr};
   void lin3(int n, double a, const double* x, double b, const double* y, double c, const double* z,
             double* out);
@@ -469,7 +470,7 @@ class DevHier {
   // is not bit-exact anyway (some level sums its rows in a tree)
   double* cinv_ = nullptr;
   bool cinv_ok_ = false;   // cinv_ is kept (such a hierarchy, n_c <= 64)
-  bool tail_inv_ = false;  // the tail applies it (n_c <= 32)
+  bool tail_inv_ = false;  // the tail applies it
   void build_cinv();
   int* info_ = nullptr;
   double *cb64_ = nullptr, *cx64_ = nullptr;

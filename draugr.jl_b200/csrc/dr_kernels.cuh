@@ -1135,15 +1135,14 @@ __device__ __forceinline__ void tail_lu_solve(const TailCoarse<T>& C) {
   const int* piv = tail_sh<const int>(C.o_piv);
   const T* cb = tail_sh<const T>(C.o_b);
   T* cx = tail_sh<T>(C.o_x);
-  if (C.inv && n <= 32) {
-    // x = A_c^-1 b, one row of the inverse per lane, summed in column order
-    if (threadIdx.x < 32) {
-      const int i = threadIdx.x;
-      if (i < n) {
-        double y = 0.0;
-        for (int j = 0; j < n; ++j) y = __dadd_rn(y, __dmul_rn(lu[j * n + i], (double)cb[j]));
-        cx[i] = (T)y;
-      }
+  if (C.inv) {
+    // x = A_c^-1 b (n <= kInvMax), one row of the inverse per thread, summed
+    // in column order
+    const int i = threadIdx.x;
+    if (i < n) {
+      double y = 0.0;
+      for (int j = 0; j < n; ++j) y = __dadd_rn(y, __dmul_rn(lu[j * n + i], (double)cb[j]));
+      cx[i] = (T)y;
     }
     __syncthreads();
     return;
@@ -1441,38 +1440,149 @@ __global__ void k_lu_factor(int n, double* __restrict__ a, int* __restrict__ piv
   }
 }
 
-// Explicit inverse of A from its getrf factors (column-major, 0-based
-// pivots), column j by thread j: A x = e_j solved in getrs order (row
-// interchanges, unit-lower then upper substitution).  n <= kInvMax.  Used
-// where the coarsest solve need not be the reference's substitutions bit for
-// bit.
+// The same factorisation with the matrix in shared memory, for n <= kInvMax:
+// the operations on every entry are k_lu_factor's, in its order, so the
+// factors are too.  Bound by the chain of n steps (a pivot search by one
+// warp and two barriers each): 42 unknowns take 43 us, 111 us in global
+// memory with a block-wide pivot search.
 constexpr int kInvMax = 64;
-__device__ __forceinline__ void lu_inverse_column(int n, const double* __restrict__ lu,
-                                                  const int* __restrict__ piv, double* __restrict__ inv,
-                                                  int j) {
-  double y[kInvMax];
-  for (int i = 0; i < n; ++i) y[i] = i == j ? 1.0 : 0.0;
-  for (int k = 0; k < n; ++k) {
-    const int p = piv[k];
-    if (p != k) {
-      const double t = y[k];
-      y[k] = y[p];
-      y[p] = t;
+constexpr int kLuThreads = 256;
+__global__ void __launch_bounds__(kLuThreads)
+k_lu_factor_small(int n, double* __restrict__ a, int* __restrict__ piv, int* info) {
+  __shared__ double s[kInvMax * (kInvMax + 1)];
+  __shared__ int sp;
+  constexpr int ld = kInvMax + 1;  // a_ij at s[j * ld + i]
+  for (int t = threadIdx.x; t < n * n; t += kLuThreads) s[t / n * ld + t % n] = a[t];
+  if (threadIdx.x == 0) *info = 0;
+  __syncthreads();
+  for (int j = 0; j < n; ++j) {
+    if (threadIdx.x < 32) {
+      // first index of the maximum magnitude in column j
+      double best = -1.0;
+      int bi = n;
+      for (int i = j + (int)threadIdx.x; i < n; i += 32) {
+        const double v = fabs(s[j * ld + i]);
+        if (v > best) { best = v; bi = i; }
+      }
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) {
+        const double v2 = __shfl_xor_sync(0xffffffffu, best, o);
+        const int i2 = __shfl_xor_sync(0xffffffffu, bi, o);
+        if (v2 > best || (v2 == best && i2 < bi)) { best = v2; bi = i2; }
+      }
+      if (threadIdx.x == 0) {
+        // every comparison fails on a column of NaNs: keep the row, as dgetf2 does
+        sp = bi < n ? bi : j;
+        piv[j] = sp;
+      }
     }
+    __syncthreads();
+    const int p = sp;
+    if (s[j * ld + p] == 0.0) {
+      if (threadIdx.x == 0) *info = j + 1;
+      break;
+    }
+    if (p != j) {
+      for (int c = threadIdx.x; c < n; c += kLuThreads) {
+        const double t = s[c * ld + j];
+        s[c * ld + j] = s[c * ld + p];
+        s[c * ld + p] = t;
+      }
+      __syncthreads();
+    }
+    // a row's multiplier is formed where it is used and stored by the
+    // thread that owns column j
+    const double r = __drcp_rn(s[j * ld + j]);
+    const int m = n - j - 1;
+    for (int t = threadIdx.x; t < m * m; t += kLuThreads) {
+      const int c = j + 1 + t / m, i = j + 1 + t % m;
+      s[c * ld + i] = __dsub_rn(s[c * ld + i], __dmul_rn(__dmul_rn(s[j * ld + i], r), s[c * ld + j]));
+    }
+    __syncthreads();
+    for (int i = j + 1 + (int)threadIdx.x; i < n; i += kLuThreads) s[j * ld + i] = __dmul_rn(s[j * ld + i], r);
   }
-  for (int k = 0; k < n; ++k)
-    if (y[k] != 0.0)
-      for (int i = k + 1; i < n; ++i) y[i] = __dsub_rn(y[i], __dmul_rn(y[k], lu[k * n + i]));
-  for (int k = n - 1; k >= 0; --k) {
-    if (y[k] != 0.0) y[k] = __ddiv_rn(y[k], lu[k * n + k]);
-    if (y[k] != 0.0)
-      for (int i = 0; i < k; ++i) y[i] = __dsub_rn(y[i], __dmul_rn(y[k], lu[k * n + i]));
-  }
-  for (int i = 0; i < n; ++i) inv[j * n + i] = y[i];
+  __syncthreads();
+  for (int t = threadIdx.x; t < n * n; t += kLuThreads) a[t] = s[t / n * ld + t % n];
 }
-__global__ void k_lu_inverse(int n, const double* __restrict__ lu, const int* __restrict__ piv,
-                             double* __restrict__ inv) {
-  if ((int)threadIdx.x < n) lu_inverse_column(n, lu, piv, inv, threadIdx.x);
+
+// Explicit inverse of A from its getrf factors (column-major, 0-based
+// pivots), n <= kInvMax: column j by one warp, A x = e_j solved in getrs order
+// (row interchanges, unit-lower then upper substitution), y_i for i = lane
+// and lane + 32 in registers and y_k passed on by shuffle.  A block of 16
+// warps walks the columns with the factors in shared memory.  Bound by the
+// chain of 2n steps: 42 unknowns take 42 us; one thread per column with y
+// in local memory took 104 us.  Used where the coarsest solve need not be the
+// reference's substitutions bit for bit.
+constexpr int kInvThreads = 512;
+__device__ __forceinline__ void lu_inverse_block(int n, const double* __restrict__ lu_g,
+                                                 const int* __restrict__ piv, double* __restrict__ inv) {
+  __shared__ double lu[kInvMax * kInvMax];
+  __shared__ int place[kInvMax], at[kInvMax];  // place[j]: where the interchanges take row j
+  for (int t = threadIdx.x; t < n * n; t += kInvThreads) lu[t] = lu_g[t];
+  if (threadIdx.x == 0) {
+    // apply the interchanges to 0 .. n-1
+    for (int i = 0; i < n; ++i) at[i] = i;
+    for (int k = 0; k < n; ++k) {
+      const int p = piv[k];
+      const int t = at[k];
+      at[k] = at[p];
+      at[p] = t;
+    }
+    for (int i = 0; i < n; ++i) place[at[i]] = i;
+  }
+  __syncthreads();
+  const int lane = threadIdx.x & 31;
+  for (int j = threadIdx.x >> 5; j < n; j += kInvThreads / 32) {
+    double y0 = lane == place[j] ? 1.0 : 0.0, y1 = lane + 32 == place[j] ? 1.0 : 0.0;
+    for (int k = 0; k < n; ++k) {
+      const double yk = __shfl_sync(0xffffffffu, k < 32 ? y0 : y1, k & 31);
+      if (yk != 0.0) {
+        if (lane > k && lane < n) y0 = __dsub_rn(y0, __dmul_rn(yk, lu[k * n + lane]));
+        if (lane + 32 > k && lane + 32 < n) y1 = __dsub_rn(y1, __dmul_rn(yk, lu[k * n + lane + 32]));
+      }
+    }
+    for (int k = n - 1; k >= 0; --k) {
+      const double d = lu[k * n + k];
+      if (lane == (k & 31)) {
+        if (k < 32) {
+          if (y0 != 0.0) y0 = __ddiv_rn(y0, d);
+        } else if (y1 != 0.0) {
+          y1 = __ddiv_rn(y1, d);
+        }
+      }
+      const double yk = __shfl_sync(0xffffffffu, k < 32 ? y0 : y1, k & 31);
+      if (yk != 0.0) {
+        if (lane < k) y0 = __dsub_rn(y0, __dmul_rn(yk, lu[k * n + lane]));
+        if (lane + 32 < k) y1 = __dsub_rn(y1, __dmul_rn(yk, lu[k * n + lane + 32]));
+      }
+    }
+    if (lane < n) inv[j * n + lane] = y0;
+    if (lane + 32 < n) inv[j * n + lane + 32] = y1;
+  }
+}
+__global__ void __launch_bounds__(kInvThreads)
+k_lu_inverse(int n, const double* __restrict__ lu, const int* __restrict__ piv, double* __restrict__ inv) {
+  lu_inverse_block(n, lu, piv, inv);
+}
+
+// x = A_c^-1 b with the explicit inverse (column-major), n <= kInvMax, one
+// thread per row summed in column order: the coarsest solve of a cycle that
+// is not the reference's bit for bit anyway (some level sums its rows in a
+// tree).  26 unknowns: about 3 us, 15.9 us by k_lu_solve's substitutions.
+template <typename T>
+__global__ void __launch_bounds__(kInvMax)
+k_inv_apply(int n, const double* __restrict__ inv, const T* __restrict__ bin, T* __restrict__ xout) {
+  __shared__ double sb[kInvMax];
+  const int i = threadIdx.x;
+  pdl_trigger();
+  pdl_wait();
+  if (i < n) sb[i] = (double)bin[i];
+  __syncthreads();
+  if (i >= n) return;
+  double y = 0.0;
+#pragma unroll 8
+  for (int j = 0; j < n; ++j) y = __dadd_rn(y, __dmul_rn(__ldg(inv + j * n + i), sb[j]));
+  xout[i] = (T)y;
 }
 
 // Scatter CSR values into a zeroed column-major dense matrix.
@@ -1497,13 +1607,40 @@ __global__ void k_invdiag(int n, const int* __restrict__ rp, const int* __restri
   }
 }
 
-// src/smoothers.jl:816-827: 1/Σ|a_ij|, or 0 if the sum is <= eps
-__global__ void k_l1_invdiag(int n, const int* __restrict__ rp, const double* __restrict__ v,
-                             double* __restrict__ invd) {
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+// src/smoothers.jl:816-827: 1/Σ|a_ij|, or 0 if the sum is <= eps.  A warp
+// takes kDiagRows rows (16, or 4 where there are few): it reads 32 entries of each at a time (coalesced, all
+// rows in flight) into shared memory, and one lane per row adds them in
+// column order.  HBM-bound on long matrices; one thread per row reading its
+// own entries took 265 us for the 7 levels of the 27-point 96^3 hierarchy,
+// 162 us this way.
+template <int kDiagRows>
+__global__ void __launch_bounds__(kBlock)
+k_l1_invdiag(int n, const int* __restrict__ rp, const double* __restrict__ v, double* __restrict__ invd) {
+  __shared__ double sv[kBlock / 32][kDiagRows][33];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const long long stride = (long long)gridDim.x * (kBlock / 32) * kDiagRows;
+  for (long long i0 = ((long long)blockIdx.x * (kBlock / 32) + w) * kDiagRows; i0 < n; i0 += stride) {
+    // lane q holds row i0 + q's bounds
+    const long long i = i0 + lane;
+    const bool mine = lane < kDiagRows && i < n;
+    const int rs = mine ? rp[i] : 0, len = mine ? rp[i + 1] - rs : 0;
+    const int longest = __reduce_max_sync(0xffffffffu, len);
     double l1 = 0.0;
-    for (int k = rp[i]; k < rp[i + 1]; ++k) l1 = __dadd_rn(l1, fabs(v[k]));
-    invd[i] = l1 > 2.220446049250313e-16 ? __drcp_rn(l1) : 0.0;
+    for (int k0 = 0; k0 < longest; k0 += 32) {
+      double t[kDiagRows];
+#pragma unroll
+      for (int q = 0; q < kDiagRows; ++q) {
+        const int s = __shfl_sync(0xffffffffu, rs, q), m = __shfl_sync(0xffffffffu, len, q);
+        t[q] = k0 + lane < m ? __ldg(v + s + k0 + lane) : 0.0;
+      }
+#pragma unroll
+      for (int q = 0; q < kDiagRows; ++q) sv[w][q][lane] = t[q];
+      __syncwarp();
+      if (mine)
+        for (int j = 0; j < min(32, len - k0); ++j) l1 = __dadd_rn(l1, fabs(sv[w][lane][j]));
+      __syncwarp();
+    }
+    if (mine) invd[i] = l1 > 2.220446049250313e-16 ? __drcp_rn(l1) : 0.0;
   }
 }
 
@@ -1909,17 +2046,15 @@ k_spgemm_warp(int nrows, const int* __restrict__ out_rp, const int* __restrict__
 // b into x, in the operation order of k_lu_solve (so each system's coarse
 // solve gives what its own hierarchy's gives).
 // The explicit inverses of the coarsest systems of a batch (block k: system
-// k, thread j: column j; inverse stored where the factors are;
+// k; inverse stored where the factors are;
 // n <= kInvMax),
 // and their application x = A^-1 b, one block of kInvMax threads per
 // system, each row of the inverse summed in column order.
-__global__ void k_lu_inverse_batch(const int* __restrict__ nb, const long long* __restrict__ luoff,
+__global__ void __launch_bounds__(kInvThreads) k_lu_inverse_batch(const int* __restrict__ nb, const long long* __restrict__ luoff,
                                    const int* __restrict__ poff, const double* __restrict__ lu_all,
                                    const int* __restrict__ piv_all, double* __restrict__ inv_all) {
   const int k = blockIdx.x;
-  const int n = nb[k];
-  if ((int)threadIdx.x < n)
-    lu_inverse_column(n, lu_all + luoff[k], piv_all + poff[k], inv_all + luoff[k], threadIdx.x);
+  lu_inverse_block(nb[k], lu_all + luoff[k], piv_all + poff[k], inv_all + luoff[k]);
 }
 
 template <typename T>
