@@ -394,7 +394,7 @@ class DevHier {
   double* bk_[8] = {nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr};
   void lin3(int n, double a, const double* x, double b, const double* y, double c, const double* z,
             double* out);
-  void precond64(const double* r, double* out, const CycleOpts& o);
+  void precond64(const double* r, double* out, const CycleOpts& o, bool fixed = false);
   void precond32(const double* r, double* out, const CycleOpts& o);  // FP32 cycle, FP64 in and out
   // batch: layout, its device arrays per merged level (coarse blocks), the
   // finest level's segment offsets and row -> segment map
@@ -424,7 +424,7 @@ class DevHier {
   // FGMRES workspace: (restart + 1) basis vectors, restart preconditioned
   // vectors, one work vector, reduction partials and tickets per column.
   int gm_m_ = 0;
-  double *gm_V_ = nullptr, *gm_Z_ = nullptr, *gm_w_ = nullptr, *gm_h_ = nullptr, *gm_part_ = nullptr;
+  double *gm_V_ = nullptr, *gm_Z_ = nullptr, *gm_w_ = nullptr, *gm_z_ = nullptr, *gm_h_ = nullptr, *gm_part_ = nullptr;
   unsigned* gm_tk_ = nullptr;
   double *ir_r_ = nullptr, *ir_d_ = nullptr, *ir_x_ = nullptr;  // iterative refinement: residual, correction, iterate
   void upload_csr(DevMat& M, int n, int m, const std::vector<int>& rp, const std::vector<int>& ci,
@@ -499,6 +499,19 @@ class DevHier {
     cudaGraphExec_t g2[2] = {nullptr, nullptr};  // preconditioner + r·z, beside it x += α p
     long long n1[2] = {0, 0}, n2[2] = {0, 0};    // kernels per graph
   } pg_;
+  // graphs of cycles on the hierarchy's own vectors (replay), at most 16; they
+  // hold device addresses only, so a resetup, which writes in place, keeps them
+  struct CycleGraph {
+    int key[6] = {0, 0, 0, 0, 0, 0};  // kind, transposed, pre, post, W, wait limit
+    const void* in = nullptr;
+    const void* out = nullptr;
+    void* result = nullptr;  // where the cycle ends
+    cudaGraphExec_t exec = nullptr;
+    long long launches = 0;  // kernels in it
+  };
+  std::vector<CycleGraph> cycle_graphs_;
+  template <class F>
+  void* replay(int kind, const void* in, void* out, const CycleOpts& o, F&& body);
   cudaEvent_t ev_[2] = {nullptr, nullptr};
   // a second stream and two events, to fork and join a branch of a graph
   // capture (the PCG iterate update beside the preconditioner)

@@ -228,10 +228,19 @@ def config_fields(config: AMGConfig | str | None) -> dict:
 
 
 _cfg_cache: dict[str, int] = {}
+_cfg_by_value: dict[AMGConfig, int] = {}  # the same handles by configuration, without writing the JSON
 
 
 def config_handle(config: AMGConfig | str | None) -> int:
     """Config handle (draugr_amg_config_from_json) for a config or JSON text."""
+    if isinstance(config, AMGConfig):
+        try:
+            h = _cfg_by_value.get(config)
+            if h is None:
+                h = _cfg_by_value[config] = config_handle(config.to_json())
+            return h
+        except TypeError:  # a field that cannot be hashed
+            pass
     js = "{}" if config is None else (config if isinstance(config, str) else config.to_json())
     h = _cfg_cache.get(js)
     if h is None:
