@@ -227,7 +227,7 @@ int resident_blocks(const void* f, int nt, size_t smem) {
 
 template <typename TA, class XL, class EP, bool DOT, class Fin>
 void launch_rows_impl(cudaStream_t st, int max_grid, const DevMat& M, const TA* av, XL xl, EP ep,
-                      double* partials, unsigned* ticket, Fin fin) {
+                      double* partials, unsigned* ticket, Fin fin, int early) {
   const RowForm& f = M.form;
   const int n = M.n, ntiles = M.ntiles;
   const int *tp = M.tp, *ts = M.ts, *tb = M.tb, *rp = M.rp, *ci = M.ci;
@@ -249,7 +249,7 @@ void launch_rows_impl(cudaStream_t st, int max_grid, const DevMat& M, const TA* 
     const int grid = std::max(                                                                   \
         1, std::min({ntiles, max_grid, g_nsm * resident_blocks((const void*)kf, NT, smem)}));    \
     launch_dependent(kf, grid, NT, smem, st, ntiles, tp, ts, tb, rp, ci, cu, av, xl, ep, partials, \
-                     ticket, fin, err_flag(), tile_wait_limit());                                \
+                     ticket, fin, err_flag(), tile_wait_limit(), early);                         \
   } while (0)
   // 16-bit column offsets where lanes read consecutive entries (flat and
   // tree forms), and for FP32 rows of 12-32 entries, where the bytes saved
@@ -269,16 +269,20 @@ void launch_rows_impl(cudaStream_t st, int max_grid, const DevMat& M, const TA* 
   DR_CK(cudaGetLastError());
 }
 
+// The row kernels read matrix values before the wait for the previous kernel
+// (`early`): every routine that writes values, diagonals of Q or their FP32
+// copies (setup, ensure_fp32, build_transpose, resetup) ends with a stream
+// synchronisation.  Launches inside a resetup pass early = 0.
 template <typename TA, class XL, class EP>
 void launch_rows(cudaStream_t st, int max_grid, const DevMat& M, const TA* av, XL xl, EP ep) {
   launch_rows_impl<TA, XL, EP, false, FinStore>(st, max_grid, M, av, xl, ep, nullptr, nullptr,
-                                                FinStore{nullptr});
+                                                FinStore{nullptr}, 1);
 }
 
 template <typename TA, class XL, class EP, class Fin>
 void launch_rows_dot(cudaStream_t st, int max_grid, const DevMat& M, const TA* av, XL xl, EP ep,
-                     double* partials, unsigned* ticket, Fin fin) {
-  launch_rows_impl<TA, XL, EP, true, Fin>(st, max_grid, M, av, xl, ep, partials, ticket, fin);
+                     double* partials, unsigned* ticket, Fin fin, int early = 1) {
+  launch_rows_impl<TA, XL, EP, true, Fin>(st, max_grid, M, av, xl, ep, partials, ticket, fin, early);
 }
 
 int grid1d(long long n, int max_grid) {
@@ -891,9 +895,8 @@ void DevHier::build_tail() {
     tail_co_[slot][2] = take(sizeof(T) * (size_t)nc_);
     tail_co_[slot][3] = take(sizeof(T) * (size_t)nc_);
     tail_bytes_[slot] = off;
-    // the prologue's bulk copies: patterns, then values, factors and the
-    // top level's right-hand side (sizes rounded up to 16 bytes; every
-    // source starts an allocation rounded the same way)
+    // the prologue's bulk copies: patterns, values and factors (sizes rounded
+    // up to 16 bytes; every source starts an allocation rounded the same way)
     std::vector<TailCopy> pat, val;
     auto rec = [&](std::vector<TailCopy>& l, unsigned o, const void* src, size_t bytes) {
       if (bytes) l.push_back(TailCopy{src, o, (unsigned)a16(bytes)});
@@ -915,17 +918,16 @@ void DevHier::build_tail() {
     }
     rec(val, tail_co_[slot][0], tail_inv_ ? cinv_ : clu_, 8 * (size_t)nc_ * nc_);
     rec(val, tail_co_[slot][1], cpiv_, 4 * (size_t)nc_);
-    rec(val, v[0].o_b, v[0].b, sizeof(T) * (size_t)v[0].n);
     TailCopyList& cl = tail_cp_[slot];
-    cl.npat = (int)pat.size();
-    cl.nval = (int)val.size();
-    cl.pat_bytes = cl.val_bytes = 0;
-    for (const TailCopy& c : pat) cl.pat_bytes += c.bytes;
-    for (const TailCopy& c : val) cl.val_bytes += c.bytes;
+    cl.bsrc = v[0].b;
+    cl.boff = v[0].o_b;
     cl.xsrc = v[0].xa;
     cl.xoff = v[0].o_xa;
     cl.xbytes = (unsigned)a16(sizeof(T) * (size_t)v[0].n);
     pat.insert(pat.end(), val.begin(), val.end());
+    cl.n = (int)pat.size();
+    cl.bytes = 0;
+    for (const TailCopy& c : pat) cl.bytes += c.bytes;
     TailCopy* dl = alloc<TailCopy>(pat.size());
     DR_CK(cudaMemcpy(dl, pat.data(), pat.size() * sizeof(TailCopy), cudaMemcpyHostToDevice));
     cl.list = dl;
@@ -1201,8 +1203,8 @@ T* DevHier::cycle_level(int l, T* x, const T* b, bool x_zero, const CycleOpts& o
                     tail_co_[slot][2], tail_co_[slot][3], tail_inv_ ? 1 : 0};
     counted();
     const TailCopyList& cl = tail_cp_[slot];
-    const TailCopies cp{static_cast<const TailCopy*>(cl.list), cl.npat, cl.nval, cl.pat_bytes,
-                        cl.val_bytes, TailCopy{cl.xsrc, cl.xoff, cl.xbytes}};
+    const TailCopies cp{static_cast<const TailCopy*>(cl.list), cl.n, cl.bytes,
+                        TailCopy{cl.bsrc, cl.boff, cl.xbytes}, TailCopy{cl.xsrc, cl.xoff, cl.xbytes}};
     launch_dependent(k_coarse_tail<T>, 1, kern::kTailThreads, tail_bytes_[slot], st_,
                      static_cast<const TailLevel<T>*>(desc), nlevels() - l, C, cp, o.pre, o.post,
                      o.w ? 1 : 0, x_zero ? 1 : 0, err_flag());
@@ -2340,7 +2342,7 @@ void DevHier::resetup_values(const double* v_dev) {
       DR_CK(cudaMemcpyAsync(v, d.cheb_v0, (size_t)d.A.n * sizeof(double), cudaMemcpyDeviceToDevice, st_));
       for (int it = 0; it < 10; ++it) {
         launch_rows_dot(st_, max_grid_, d.A, d.A.v, XPlain<double>{v}, EpPowerStep{d.invd, w}, partials_,
-                        tickets_ + TK_DOT, FinStore{lam2});
+                        tickets_ + TK_DOT, FinStore{lam2}, 0);  // this resetup wrote the values
         counted();
         k_cheb_rescale<<<grid1d(d.A.n, max_grid_), kBlock, 0, st_>>>(d.A.n, w, lam2, v);
       }

@@ -442,10 +442,10 @@ class DevHier {
   size_t tail_bytes_[2] = {0, 0};        // shared memory of the tail kernel (FP64, FP32)
   struct TailCopyList {  // its prologue's bulk copies (kern::TailCopies)
     const void* list = nullptr;
-    int npat = 0, nval = 0;
-    unsigned pat_bytes = 0, val_bytes = 0;
-    const void* xsrc = nullptr;
-    unsigned xoff = 0, xbytes = 0;
+    int n = 0;
+    unsigned bytes = 0;
+    const void *bsrc = nullptr, *xsrc = nullptr;  // the top level's right-hand side and iterate
+    unsigned boff = 0, xoff = 0, xbytes = 0;
   } tail_cp_[2];
   unsigned tail_co_[2][4] = {{0}, {0}};  // its coarsest-system offsets (TailCoarse)
   void graphs_clear();

@@ -502,7 +502,7 @@ __global__ void __launch_bounds__(NT, (tile_min_blocks<NT, TA>()))
 k_tile_rows(int ntiles, const int* __restrict__ tp, const int* __restrict__ ts,
             const int* __restrict__ tb, const int* __restrict__ rp, const int* __restrict__ ci,
             const uint16_t* __restrict__ cu, const TA* __restrict__ av, XL xl, EP ep,
-            double* partials, unsigned* ticket, Fin fin, int* err, int wait_limit) {
+            double* partials, unsigned* ticket, Fin fin, int* err, int wait_limit, int early) {
   constexpr bool kOff = sizeof(TC) == 2;
   constexpr int kColAlign = 16 / (int)sizeof(TC);  // entries per 16 bytes
   const TC* const csrc = kOff ? reinterpret_cast<const TC*>(cu) : reinterpret_cast<const TC*>(ci);
@@ -589,18 +589,26 @@ k_tile_rows(int ntiles, const int* __restrict__ tp, const int* __restrict__ ts,
   // thread's row bounds and epilogue operands of tile t + stride are in
   // flight to registers, and so are the bounds of tile t + 2 stride.  What
   // is left on a tile's critical path is the L2 gather of x.
-  // Up to pdl_wait() only the pattern is read (it never changes).
+  // Up to pdl_wait() only the pattern is read, which never changes, and with
+  // `early` the matrix values, which then no kernel in flight writes: a level
+  // of a few thousand rows is then left with one gather of x between the
+  // previous kernel's end and its own (the 2-D 300^2 FGMRES solve, 139 cycles
+  // on 12 levels: 25.6 ms with the values requested after the wait, 25.1 before; 128^3 cycle 599 and 584 us).
   Head h0 = head(blockIdx.x), h1 = head(blockIdx.x + stride);
   if (threadIdx.x == 0) {
     if (blockIdx.x < ntiles) issue_cols(h0, 0);
     if (blockIdx.x + stride < ntiles) issue_cols(h1, 1);
+    if (early) {
+      if (blockIdx.x < ntiles) issue_vals(h0, 0);
+      if (blockIdx.x + stride < ntiles) issue_vals(h1, 1);
+    }
   }
   Ctx c0 = ctx_rows(h0);
   pdl_trigger();
   pdl_wait();
   bind_loader(xl);
   bind_epilogue(ep);
-  if (threadIdx.x == 0) {
+  if (!early && threadIdx.x == 0) {
     if (blockIdx.x < ntiles) issue_vals(h0, 0);
     if (blockIdx.x + stride < ntiles) issue_vals(h1, 1);
   }
@@ -1019,14 +1027,14 @@ struct TailCopy {
   unsigned off, bytes;
 };
 
-// The tail's copies: pattern arrays first (never written by a kernel),
-// then the rest; x, the top level's iterate, is copied only when the
-// visit does not start from zero.
+// The tail's copies: the levels' patterns and values and the coarsest factors
+// (written by no kernel in flight), then the top level's right-hand side; x,
+// its iterate, is copied only when the visit does not start from zero.
 struct TailCopies {
   const TailCopy* list;
-  int npat, nval;
-  unsigned pat_bytes, val_bytes;
-  TailCopy x;
+  int n;
+  unsigned bytes;
+  TailCopy b, x;
 };
 
 // a ± Σ_k v[k]·x[c[k]] over [s, e) in column order.  Eight entries at a
@@ -1311,27 +1319,24 @@ k_coarse_tail(const TailLevel<T>* __restrict__ lv, int nl, TailCoarse<T> C, Tail
     if (threadIdx.x == 0) {
       mbar_init(&bar, 1);
       fence_mbar_init();
-      mbar_expect_tx(&bar, cp.pat_bytes + cp.val_bytes + (x_zero ? 0u : cp.x.bytes));
+      mbar_expect_tx(&bar, cp.bytes + cp.b.bytes + (x_zero ? 0u : cp.x.bytes));
     }
     __syncwarp();
-    for (int i = threadIdx.x; i < cp.npat; i += 32) {
+    for (int i = threadIdx.x; i < cp.n; i += 32) {
       const TailCopy c = cp.list[i];
       bulk_g2s(tsm + c.off, c.src, c.bytes, &bar);
     }
-  }
-  pdl_trigger();
-  pdl_wait();
-  if (threadIdx.x < 32) {
-    for (int i = threadIdx.x; i < cp.nval; i += 32) {
-      const TailCopy c = cp.list[cp.npat + i];
-      bulk_g2s(tsm + c.off, c.src, c.bytes, &bar);
-    }
-    if (threadIdx.x == 0 && !x_zero && cp.x.bytes) bulk_g2s(tsm + cp.x.off, cp.x.src, cp.x.bytes, &bar);
   }
   // the descriptors (sizes, ω, shared-memory offsets) into shared memory
   if (threadIdx.x < nl) sl[threadIdx.x] = lv[threadIdx.x];
   if (threadIdx.x == 32) sc = C;
   if (threadIdx.x == 0) ok = 1;
+  pdl_trigger();
+  pdl_wait();
+  if (threadIdx.x == 0) {
+    if (cp.b.bytes) bulk_g2s(tsm + cp.b.off, cp.b.src, cp.b.bytes, &bar);
+    if (!x_zero && cp.x.bytes) bulk_g2s(tsm + cp.x.off, cp.x.src, cp.x.bytes, &bar);
+  }
   __syncthreads();  // barrier initialised, descriptors published
   if (!mbar_wait_bounded(&bar, 0, kWaitLimit)) ok = 0;  // every thread observes the copies
   __syncthreads();
