@@ -566,6 +566,8 @@ DevHier::~DevHier() {
   if (seg_graph_) cudaGraphExecDestroy(seg_graph_);
   for (void* p : allocs_) cudaFree(p);
   if (hscal_) cudaFreeHost(hscal_);
+  if (bi_host_) cudaFreeHost(bi_host_);
+  if (gm_host_) cudaFreeHost(gm_host_);
   cudaEventDestroy(ev_[0]);
   cudaEventDestroy(ev_[1]);
   if (ev_fork_) cudaEventDestroy(ev_fork_);
@@ -617,6 +619,12 @@ void DevHier::graphs_clear() {
 // single launches, 49.9 with graphs; a 2256-row 2-D cycle: 181 and 149 us).
 template <class F>
 void* DevHier::replay(int kind, const void* in, void* out, const CycleOpts& o, F&& body) {
+  if (in_replay_) return body();  // part of a larger graph
+  struct Flag {
+    bool& f;
+    ~Flag() { f = false; }
+  } flag{in_replay_};
+  in_replay_ = true;
   const int key[6] = {kind, tr_ ? 1 : 0, o.pre, o.post, o.w ? 1 : 0, tile_wait_limit()};
   CycleGraph* g = nullptr;
   for (CycleGraph& c : cycle_graphs_)
@@ -1176,7 +1184,10 @@ void DevHier::coarse_solve(const T* b, T* x, bool inverse_allowed) {
   const int staged = (ybytes + lbytes) <= 40 * 1024 ? 1 : 0;
   counted();
   if (tr_) {  // A_c^T y = b with the factors of A_c (adjoint solves)
-    k_lu_solve_t<T><<<1, 32, ybytes, st_>>>(nc_, clu_, cpiv_, b, x);
+    if (nc_ <= 64)
+      launch_dependent(k_lu_solve_t_warp<T>, 1, 32, 0, st_, nc_, (const double*)clu_, (const int*)cpiv_, b, x);
+    else
+      k_lu_solve_t<T><<<1, 32, ybytes, st_>>>(nc_, clu_, cpiv_, b, x);
     DR_CK(cudaGetLastError());
     return;
   }
@@ -1490,12 +1501,18 @@ int DevHier::bicgstab(double* x, const double* b, const CycleOpts& o, double tol
   } mode{tr_, tr_};
   tr_ = transpose;
   const int n = n0_;
-  if (!bk_[0])
+  if (!bk_[0]) {
     for (auto& p : bk_) p = alloc<double>(n);
+    bi_scal_ = alloc<double>(BS_N);
+    bi_part_ = alloc<double>(2 * (size_t)max_grid_);
+    DR_CK(cudaMallocHost(&bi_host_, 2 * BS_N * sizeof(double)));
+  }
   double *r = bk_[0], *rh = bk_[1], *p = bk_[2], *v = bk_[3], *sv = bk_[4], *t = bk_[5], *ph = bk_[6],
          *sh = bk_[7];
+  double* S = bi_scal_;
+  double* const xout = x;
+  const DevMat& A = L_.empty() ? C_ : (tr_ ? L_[0].At : L_[0].A);
   auto spmv = [&](const double* in, double* out) {
-    const DevMat& A = L_.empty() ? C_ : (tr_ ? L_[0].At : L_[0].A);
     launch_rows(st_, max_grid_, A, A.v, XPlain<double>{in}, EpStore<double>{out});
   };
   const double bnorm = std::sqrt(dot_host(b, b, n));
@@ -1506,50 +1523,84 @@ int DevHier::bicgstab(double* x, const double* b, const CycleOpts& o, double tol
     if (relres) *relres = 0.0;
     return 0;
   }
+  // the iterate in the hierarchy's own vector
+  x = xd_;
+  if (xout != x) DR_CK(cudaMemcpyAsync(x, xout, (size_t)n * sizeof(double), cudaMemcpyDeviceToDevice, st_));
   spmv(x, t);
   lin3(n, 1.0, b, -1.0, t, 0.0, nullptr, r);  // r = b - A x
   DR_CK(cudaMemcpyAsync(rh, r, (size_t)n * sizeof(double), cudaMemcpyDeviceToDevice, st_));
-  double rel = std::sqrt(dot_host(r, r, n)) / bnorm;
-  double rho = 1.0, alpha = 1.0, omega = 1.0;
+  double rho1 = dot_host(r, r, n);  // rh·r, and r·r
+  double rel = std::sqrt(rho1) / bnorm;
   counted();
   k_fill<double><<<grid1d(n, max_grid_), kBlock, 0, st_>>>(n, 0.0, p);
   counted();
   k_fill<double><<<grid1d(n, max_grid_), kBlock, 0, st_>>>(n, 0.0, v);
+  {
+    double* h = bi_host_;
+    for (int i = 0; i < BS_N; ++i) h[i] = 0.0;
+    h[BS_RHO] = h[BS_ALPHA] = h[BS_OMEGA] = 1.0;
+    h[BS_RHO1] = rho1;
+    h[BS_BNORM] = bnorm;
+    h[BS_TOL] = tol;
+    DR_CK(cudaMemcpyAsync(S, h, BS_N * sizeof(double), cudaMemcpyHostToDevice, st_));
+    DR_CK(cudaStreamSynchronize(st_));
+  }
+  const int gx = grid1d(n, max_grid_);
+  // One iteration, as one graph, its scalars copied to pinned slot `par` at
+  // its end.  The next iteration is enqueued before the host reads them; if
+  // the solve has stopped by then, that one changes neither x nor r.
+  auto iteration = [&](int par) {
+    double* slot = bi_host_ + par * BS_N;
+    replay((mixed ? 6 : 4) + par, slot, x, o, [&]() -> void* {
+      counted();
+      launch_dependent(k_bicg_p, gx, kBlock, 0, st_, n, (const double*)S, (const double*)r, (const double*)v, p);
+      if (mixed) precond32(p, ph, o);
+      else precond64(p, ph, o);
+      launch_rows_dot(st_, max_grid_, A, A.v, XPlain<double>{ph}, EpStoreDot{v, rh}, partials_, tickets_ + TK_DOT,
+                      FinStore{S + BS_RHV});
+      counted();
+      launch_dependent(k_bicg_s, gx, kBlock, 0, st_, n, S, (const double*)r, (const double*)v, sv, bi_part_,
+                       tickets_ + TK_RES);
+      if (mixed) precond32(sv, sh, o);
+      else precond64(sv, sh, o);
+      launch_rows_dot(st_, max_grid_, A, A.v, XPlain<double>{sh}, EpStoreDot{t, sv}, partials_, tickets_ + TK_DOT,
+                      FinStore{S + BS_TS});
+      counted();
+      k_dot<double, double, FinStore><<<gx, kBlock, 0, st_>>>(n, t, t, partials_, tickets_ + TK_DOT,
+                                                             FinStore{S + BS_TT});
+      counted();
+      launch_dependent(k_bicg_x, gx, kBlock, 0, st_, n, S, (const double*)ph, (const double*)sh, (const double*)sv,
+                       (const double*)t, (const double*)rh, x, r, bi_part_, tickets_ + TK_RES);
+      DR_CK(cudaMemcpyAsync(slot, S, BS_N * sizeof(double), cudaMemcpyDeviceToHost, st_));
+      return x;
+    });
+    DR_CK(cudaEventRecord(ev_[par], st_));
+  };
   int it = 0;
-  while (rel >= tol && it < maxiter) {
-    ++it;
-    const double rho1 = dot_host(rh, r, n);
-    if (rho1 == 0.0) break;  // breakdown: r orthogonal to the shadow residual
-    const double beta = (rho1 / rho) * (alpha / omega);
-    lin3(n, 1.0, r, beta, p, -beta * omega, v, p);  // p = r + beta (p - omega v)
-    if (mixed) precond32(p, ph, o);
-    else precond64(p, ph, o, true);
-    spmv(ph, v);
-    alpha = rho1 / dot_host(rh, v, n);
-    lin3(n, 1.0, r, -alpha, v, 0.0, nullptr, sv);  // s = r - alpha v
-    const double snorm = std::sqrt(dot_host(sv, sv, n));
-    if (snorm / bnorm < tol) {
-      lin3(n, 1.0, x, alpha, ph, 0.0, nullptr, x);
-      DR_CK(cudaMemcpyAsync(r, sv, (size_t)n * sizeof(double), cudaMemcpyDeviceToDevice, st_));
-      rel = snorm / bnorm;
-      break;
+  if (rel >= tol && maxiter > 0) {
+    iteration(0);
+    while (true) {
+      ++it;
+      if (rho1 == 0.0) break;  // breakdown: r orthogonal to the shadow residual
+      if (it < maxiter) iteration(it & 1);
+      DR_CK(cudaEventSynchronize(ev_[(it - 1) & 1]));
+      const double* h = bi_host_ + ((it - 1) & 1) * BS_N;
+      const double srel = std::sqrt(h[BS_SS]) / bnorm;
+      if (srel < tol) {  // met at the half step
+        rel = srel;
+        break;
+      }
+      rel = std::sqrt(h[BS_RR]) / bnorm;
+      rho1 = h[BS_RHO1];
+      if (verbose >= 2) std::printf("  BiCGStab iter %4d: relative residual %.6e\n", it, rel);
+      if (h[BS_OMEGA] == 0.0 || !(rel >= tol) || it >= maxiter) break;
     }
-    if (mixed) precond32(sv, sh, o);
-    else precond64(sv, sh, o, true);
-    spmv(sh, t);
-    const double tt = dot_host(t, t, n);
-    omega = tt > 0.0 ? dot_host(t, sv, n) / tt : 0.0;
-    lin3(n, 1.0, x, alpha, ph, omega, sh, x);      // x += alpha p^ + omega s^
-    lin3(n, 1.0, sv, -omega, t, 0.0, nullptr, r);  // r = s - omega t
-    rel = std::sqrt(dot_host(r, r, n)) / bnorm;
-    rho = rho1;
-    if (verbose >= 2) std::printf("  BiCGStab iter %4d: relative residual %.6e\n", it, rel);
-    if (omega == 0.0) break;
   }
   // true residual of the result
   spmv(x, t);
   lin3(n, 1.0, b, -1.0, t, 0.0, nullptr, r);
   rel = std::sqrt(dot_host(r, r, n)) / bnorm;
+  if (xout != x) DR_CK(cudaMemcpyAsync(xout, x, (size_t)n * sizeof(double), cudaMemcpyDeviceToDevice, st_));
   check_kernel_flag(st_, hscal_);
   if (relres) *relres = rel;
   return it;
@@ -1585,6 +1636,8 @@ void DevHier::precond32(const double* r, double* out, const CycleOpts& o) {
 // on the host (one device-to-host copy per iteration).  Restarts from the
 // true residual; stops when the rotated residual estimate, and then the true
 // residual, is below tol·||b||.
+static constexpr int kHess = 2 * 64 + 2;  // a step's two Gram-Schmidt columns and the norm
+
 int DevHier::fgmres(double* x, const double* b, const CycleOpts& o, double tol, int maxiter, int restart,
                     bool mixed, double* relres, int verbose) {
   const int n = n0_;
@@ -1597,8 +1650,9 @@ int DevHier::fgmres(double* x, const double* b, const CycleOpts& o, double tol, 
     gm_Z_ = alloc<double>((size_t)m * n);
     gm_w_ = alloc<double>(n);
     if (!gm_z_) gm_z_ = alloc<double>(n);
-    gm_h_ = alloc<double>(2 * 64 + 2);
+    gm_h_ = alloc<double>(kHess);
     gm_part_ = alloc<double>((size_t)65 * max_grid_);
+    if (!gm_host_) DR_CK(cudaMallocHost(&gm_host_, 2 * kHess * sizeof(double)));
     gm_tk_ = alloc<unsigned>(65);
     DR_CK(cudaMemsetAsync(gm_tk_, 0, 65 * sizeof(unsigned), st_));
     gm_m_ = m;
@@ -1610,7 +1664,9 @@ int DevHier::fgmres(double* x, const double* b, const CycleOpts& o, double tol, 
   };
   auto mdot = [&](int k, const double* vw, double* h) {
     counted();
-    k_mdot<<<dim3(gx, k), kBlock, 0, st_>>>(n, V, (long long)n, vw, gm_part_, gm_tk_, h);
+    // about one wave of blocks over all columns (352 blocks of 256 rows for
+    // each of 30 columns took 12 us at 90 k rows, 5.8 us this way)
+    k_mdot<<<dim3(std::max(1, std::min(gx, max_grid_ / k)), k), kBlock, 0, st_>>>(n, V, (long long)n, vw, gm_part_, gm_tk_, h);
   };
   auto maxpy = [&](int k, const double* Mv, const double* h, double sign, double* out) {
     counted();
@@ -1624,7 +1680,7 @@ int DevHier::fgmres(double* x, const double* b, const CycleOpts& o, double tol, 
     if (relres) *relres = 0.0;
     return 0;
   }
-  std::vector<double> H((size_t)(m + 1) * m), cs(m), sn(m), g(m + 1), y(m), hh(2 * 64 + 2);
+  std::vector<double> H((size_t)(m + 1) * m), cs(m), sn(m), g(m + 1), y(m);
   int it = 0;
   double rel = 1.0;
   while (true) {
@@ -1638,8 +1694,11 @@ int DevHier::fgmres(double* x, const double* b, const CycleOpts& o, double tol, 
     std::fill(g.begin(), g.end(), 0.0);
     g[0] = beta;
     int jn = 0;  // columns in this cycle
-    for (int j = 0; j < m && it < maxiter; ++j) {
-      ++it;
+    // Everything of step j, its Hessenberg column copied to pinned slot j & 1
+    // at the end.  Step j + 1 is enqueued before the host waits for step j's
+    // column, so the GPU does not idle between steps; a step past the last one
+    // needed writes only vectors that are not used.
+    auto step = [&](int j) {
       double* vj = V + (size_t)j * n;
       double* zj = Z + (size_t)j * n;
       if (mixed) precond32(vj, zj, o);
@@ -1660,14 +1719,22 @@ int DevHier::fgmres(double* x, const double* b, const CycleOpts& o, double tol, 
       counted();
       k_dot<double, double, FinStore><<<gx, kBlock, 0, st_>>>(n, w, w, partials_, tickets_ + TK_DOT,
                                                              FinStore{gm_h_ + 128});
+      counted();
+      k_normalize<<<gx, kBlock, 0, st_>>>(n, w, gm_h_ + 128, V + (size_t)(j + 1) * n);
       DR_CK(cudaGetLastError());
-      DR_CK(cudaMemcpyAsync(hh.data(), gm_h_, hh.size() * sizeof(double), cudaMemcpyDeviceToHost, st_));
-      DR_CK(cudaStreamSynchronize(st_));
+      DR_CK(cudaMemcpyAsync(gm_host_ + (j & 1) * kHess, gm_h_, kHess * sizeof(double), cudaMemcpyDeviceToHost, st_));
+      DR_CK(cudaEventRecord(ev_[j & 1], st_));
+    };
+    step(0);
+    for (int j = 0; j < m && it < maxiter; ++j) {
+      ++it;
+      if (j + 1 < m && it < maxiter) step(j + 1);
+      DR_CK(cudaEventSynchronize(ev_[j & 1]));
+      const double* hh = gm_host_ + (j & 1) * kHess;
       const double hn = std::sqrt(hh[128]);
       double* col = &H[(size_t)j * (m + 1)];
       for (int i = 0; i <= j; ++i) col[i] = hh[i] + hh[64 + i];
       col[j + 1] = hn;
-      if (hn > 0.0) lin3(n, 1.0 / hn, w, 0.0, w, 0.0, nullptr, V + (size_t)(j + 1) * n);
       // previous rotations, then a new one zeroing col[j+1]
       for (int i = 0; i < j; ++i) {
         const double t = cs[i] * col[i] + sn[i] * col[i + 1];

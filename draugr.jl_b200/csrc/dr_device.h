@@ -392,6 +392,8 @@ class DevHier {
   void refresh_transpose();
   void l1_invdiag(const DevMat& M, double* invd);
   double* bk_[8] = {nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr};
+  double *bi_scal_ = nullptr, *bi_part_ = nullptr;  // BiCGStab scalars and partial sums
+  double* bi_host_ = nullptr;                      // pinned, two copies of the scalars
   void lin3(int n, double a, const double* x, double b, const double* y, double c, const double* z,
             double* out);
   void precond64(const double* r, double* out, const CycleOpts& o, bool fixed = false);
@@ -426,6 +428,7 @@ class DevHier {
   int gm_m_ = 0;
   double *gm_V_ = nullptr, *gm_Z_ = nullptr, *gm_w_ = nullptr, *gm_z_ = nullptr, *gm_h_ = nullptr, *gm_part_ = nullptr;
   unsigned* gm_tk_ = nullptr;
+  double* gm_host_ = nullptr;  // pinned, two Hessenberg columns
   double *ir_r_ = nullptr, *ir_d_ = nullptr, *ir_x_ = nullptr;  // iterative refinement: residual, correction, iterate
   void upload_csr(DevMat& M, int n, int m, const std::vector<int>& rp, const std::vector<int>& ci,
                   const std::vector<double>* v);
@@ -510,6 +513,7 @@ class DevHier {
     long long launches = 0;  // kernels in it
   };
   std::vector<CycleGraph> cycle_graphs_;
+  bool in_replay_ = false;
   template <class F>
   void* replay(int kind, const void* in, void* out, const CycleOpts& o, F&& body);
   cudaEvent_t ev_[2] = {nullptr, nullptr};
