@@ -39,7 +39,7 @@ __device__ __forceinline__ float rn_add(float a, float b) { return __fadd_rn(a, 
 __device__ __forceinline__ double rn_sub(double a, double b) { return __dsub_rn(a, b); }
 __device__ __forceinline__ float rn_sub(float a, float b) { return __fsub_rn(a, b); }
 
-enum : int { BM_STORE = 0, BM_RESID = 1, BM_JACOBI = 2, BM_ADDTO = 3, BM_CORRECT = 4 };
+enum : int { BM_STORE = 0, BM_RESID = 1, BM_JACOBI = 2, BM_ADDTO = 3, BM_CORRECT = 4, BM_JZRES = 5 };
 
 // Y = A X (STORE), Y = B - A X (RESID), Y = X + (omega d)(B - A X)
 // (JACOBI), Y += A X (ADDTO, A = P), Y = Y + (omega d) B + A X (CORRECT:
@@ -139,29 +139,41 @@ __device__ __forceinline__ void block_col_partials(const double (&s)[V], int k, 
 }
 
 // With `part` (STORE mode), also the column partials of X_row . Y_row (the
-// p . q of block CG).
-template <typename TA, typename T, int MODE, int TPR>
+// p . q of block CG).  JZRES: the first Jacobi step from a zero iterate and the
+// residual after it in one pass, Y1 = (omega d) B, Y = B - A Y1, with Y1's
+// entries formed from B where they are gathered (the separate kernel wrote and
+// read n x k values more: 72 of 181 us on the finest level at 96^3 x 32).  STORE
+// with Y1 (a restriction) also writes the coarse level's first step
+// Y1 = (omega d) Y.
+//
+// SPLIT: one row per warp, its entries dealt to the 32 / TPR groups of lanes in
+// runs of TPR, the groups' sums added by a fixed shuffle tree.  For long rows
+// on levels too small to fill the GPU with TPR lanes per row, where one group
+// walked a row of hundreds of entries one L2 round trip per 4 (2843 rows of
+// 161 entries: 76 us per residual, 34 us split).
+template <typename TA, typename T, int MODE, int TPR, bool SPLIT>
 __global__ void __launch_bounds__(kBlock)
 k_spmm_vec(int nrows, int k, const int* __restrict__ rp, const int* __restrict__ ci,
            const TA* __restrict__ av, const T* __restrict__ X, const T* __restrict__ B,
-           const T* __restrict__ dinv, T omega, T* Y, double* __restrict__ part) {
+           const T* __restrict__ dinv, T omega, T* Y, T* __restrict__ Y1, double* __restrict__ part) {
   using VV = VecPiece<T>;
   using VT = typename VV::type;
   constexpr int V = VV::V;
-  constexpr int RPW = 32 / TPR;
+  constexpr int RPW = SPLIT ? 1 : 32 / TPR;
   const int lane = threadIdx.x & 31;
   const int sub = lane % TPR;
+  const int grp = lane / TPR;
   const int c0 = sub * V;           // first column of this thread
   const bool act = c0 < k;
   const int cg = act ? c0 : k - V;  // lanes past k read (and drop) the last piece
-  // the TPR lanes of one row (a row's lanes always run together)
+  // the TPR lanes of one group (a group's lanes always run together)
   const unsigned gmask = TPR == 32 ? 0xffffffffu : (((1u << TPR) - 1u) << (lane & ~(TPR - 1)));
   double dsum[V];
 #pragma unroll
   for (int q = 0; q < V; ++q) dsum[q] = 0.0;
   const long long w = (long long)blockIdx.x * kWarps + (threadIdx.x >> 5);
   const long long nw = (long long)gridDim.x * kWarps;
-  for (long long r = w * RPW + lane / TPR; r < nrows; r += nw * RPW) {
+  for (long long r = w * RPW + (SPLIT ? 0 : grp); r < nrows; r += nw * RPW) {
     const int row = (int)r;
     const int rs = rp[row], re = rp[row + 1];
     const size_t o = (size_t)row * k + cg;
@@ -178,22 +190,32 @@ k_spmm_vec(int nrows, int k, const int* __restrict__ rp, const int* __restrict__
     } else
 #pragma unroll
       for (int q = 0; q < V; ++q) acc[q] = T(0);
-    // the row's lanes load up to TPR (column, value) pairs at once and pass
+    T base[V];  // SPLIT: what the row's sum is added to (subtracted from)
+    if (SPLIT)
+#pragma unroll
+      for (int q = 0; q < V; ++q) {
+        base[q] = acc[q];
+        acc[q] = T(0);
+      }
+    // the group's lanes load up to TPR (column, value) pairs at once and pass
     // them round; the X pieces of 4 entries are gathered before the first
     // is used (slots past the row's end repeat its last entry)
-    for (int k0 = rs; k0 < re; k0 += TPR) {
+    for (int k0 = rs + (SPLIT ? grp * TPR : 0); k0 < re; k0 += SPLIT ? 32 : TPR) {
       const int my = k0 + sub;
       const int cj = my < re ? ci[my] : 0;
       const T vj = my < re ? (T)av[my] : T(0);
+      T wj = T(0);
+      if (MODE == BM_JZRES && my < re) wj = rn_mul(omega, dinv[cj]);
       const int cnt = min(TPR, re - k0);
       for (int j0 = 0; j0 < cnt; j0 += 4) {
-        T vv[4];
+        T vv[4], ww[4];
         VT xs[4];
 #pragma unroll
         for (int u = 0; u < 4; ++u) {
           const int jj = min(j0 + u, cnt - 1);
           const int c = __shfl_sync(gmask, cj, jj, TPR);
           vv[u] = __shfl_sync(gmask, vj, jj, TPR);
+          if (MODE == BM_JZRES) ww[u] = __shfl_sync(gmask, wj, jj, TPR);
           xs[u] = *reinterpret_cast<const VT*>(X + (size_t)c * k + cg);
         }
 #pragma unroll
@@ -203,19 +225,36 @@ k_spmm_vec(int nrows, int k, const int* __restrict__ rp, const int* __restrict__
             VV::get(xs[u], xv);
 #pragma unroll
             for (int q = 0; q < V; ++q) {
-              const T p = rn_mul(vv[u], xv[q]);
-              acc[q] = (MODE == BM_JACOBI) ? rn_sub(acc[q], p) : rn_add(acc[q], p);
+              const T p = rn_mul(vv[u], MODE == BM_JZRES ? rn_mul(ww[u], xv[q]) : xv[q]);
+              acc[q] = (MODE == BM_JACOBI && !SPLIT) ? rn_sub(acc[q], p) : rn_add(acc[q], p);
             }
           }
       }
     }
-    if (!act) continue;
+    if (SPLIT) {
+      __syncwarp();
+#pragma unroll
+      for (int off = TPR; off < 32; off <<= 1)
+#pragma unroll
+        for (int q = 0; q < V; ++q) acc[q] = rn_add(acc[q], __shfl_xor_sync(0xffffffffu, acc[q], off));
+#pragma unroll
+      for (int q = 0; q < V; ++q)
+        acc[q] = MODE == BM_JACOBI ? rn_sub(base[q], acc[q]) : rn_add(base[q], acc[q]);
+    }
+    if (!act || (SPLIT && grp != 0)) continue;
     T out[V];
-    if (MODE == BM_RESID) {
+    if (MODE == BM_RESID || MODE == BM_JZRES) {
       T bv[V];
       VV::get(*reinterpret_cast<const VT*>(B + o), bv);
 #pragma unroll
       for (int q = 0; q < V; ++q) out[q] = rn_sub(bv[q], acc[q]);
+      if (MODE == BM_JZRES) {
+        T x1[V];
+        const T sc = rn_mul(omega, dinv[row]);
+#pragma unroll
+        for (int q = 0; q < V; ++q) x1[q] = rn_mul(sc, bv[q]);
+        *reinterpret_cast<VT*>(Y1 + o) = VV::make(x1);
+      }
     } else if (MODE == BM_JACOBI) {
       T xo[V];
       VV::get(*reinterpret_cast<const VT*>(X + o), xo);
@@ -227,6 +266,13 @@ k_spmm_vec(int nrows, int k, const int* __restrict__ rp, const int* __restrict__
       for (int q = 0; q < V; ++q) out[q] = acc[q];
     }
     *reinterpret_cast<VT*>(Y + o) = VV::make(out);
+    if (MODE == BM_STORE && Y1) {
+      T x1[V];
+      const T sc = rn_mul(omega, dinv[row]);
+#pragma unroll
+      for (int q = 0; q < V; ++q) x1[q] = rn_mul(sc, out[q]);
+      *reinterpret_cast<VT*>(Y1 + o) = VV::make(x1);
+    }
     if (MODE == BM_STORE && part) {
       T xo[V];
       VV::get(*reinterpret_cast<const VT*>(X + o), xo);
@@ -237,14 +283,13 @@ k_spmm_vec(int nrows, int k, const int* __restrict__ rp, const int* __restrict__
   if (MODE == BM_STORE && part) block_col_partials<TPR, V>(dsum, k, part);
 }
 
-// X += alpha_c P, R -= alpha_c Q, optionally R32 = (float) R, and the
-// column partials of R . R; vector layout (TPR threads per row, 2 columns
-// per thread).
+// R -= alpha_c Q, optionally R32 = (float) R, and the column partials of R . R;
+// vector layout (TPR threads per row, 2 columns per thread).  X += alpha_c P
+// follows in k_bl_dirx, which reads P anyway.
 template <int TPR>
 __global__ void __launch_bounds__(kBlock)
-k_bl_update_vec(int n, int k, const double* __restrict__ alpha, double* __restrict__ X,
-                double* __restrict__ R, const double* __restrict__ P, const double* __restrict__ Q,
-                float* __restrict__ R32, double* __restrict__ part) {
+k_bl_update_vec(int n, int k, const double* __restrict__ alpha, double* __restrict__ R,
+                const double* __restrict__ Q, float* __restrict__ R32, double* __restrict__ part) {
   constexpr int RPW = 32 / TPR;
   const int lane = threadIdx.x & 31;
   const int c0 = (lane % TPR) * 2;
@@ -255,15 +300,10 @@ k_bl_update_vec(int n, int k, const double* __restrict__ alpha, double* __restri
   const long long nw = (long long)gridDim.x * kWarps;
   for (long long r = w * RPW + lane / TPR; act && r < n; r += nw * RPW) {
     const size_t o = (size_t)r * k + c0;
-    double2 x = *reinterpret_cast<const double2*>(X + o);
     double2 rr = *reinterpret_cast<const double2*>(R + o);
-    const double2 p = *reinterpret_cast<const double2*>(P + o);
     const double2 q = *reinterpret_cast<const double2*>(Q + o);
-    x.x += a0 * p.x;
-    x.y += a1 * p.y;
     rr.x = rr.x - a0 * q.x;
     rr.y = rr.y - a1 * q.y;
-    *reinterpret_cast<double2*>(X + o) = x;
     *reinterpret_cast<double2*>(R + o) = rr;
     if (R32) *reinterpret_cast<float2*>(R32 + o) = make_float2((float)rr.x, (float)rr.y);
     s[0] += rr.x * rr.x;
@@ -272,8 +312,8 @@ k_bl_update_vec(int n, int k, const double* __restrict__ alpha, double* __restri
   block_col_partials<TPR, 2>(s, k, part);
 }
 
-// Z = (double) z and the column partials of R . Z (the preconditioned
-// residual handed back to block CG); vector layout, 2 columns per thread.
+// The column partials of R . z, z the preconditioned residual, and with Z set
+// Z = (double) z (the first direction); vector layout, 2 columns per thread.
 template <typename TS, int TPR>
 __global__ void __launch_bounds__(kBlock)
 k_bl_take_z(int n, int k, const TS* __restrict__ z, const double* __restrict__ R, double* __restrict__ Z,
@@ -289,7 +329,7 @@ k_bl_take_z(int n, int k, const TS* __restrict__ z, const double* __restrict__ R
     const size_t o = (size_t)r * k + c0;
     const double z0 = (double)z[o], z1 = (double)z[o + 1];
     const double2 rr = *reinterpret_cast<const double2*>(R + o);
-    *reinterpret_cast<double2*>(Z + o) = make_double2(z0, z1);
+    if (Z) *reinterpret_cast<double2*>(Z + o) = make_double2(z0, z1);
     s[0] += rr.x * z0;
     s[1] += rr.y * z1;
   }
@@ -492,6 +532,30 @@ __global__ void k_bl_dir(int n, int k, const double* __restrict__ beta, const do
     P[e] = Z[e] + beta[e % k] * P[e];
 }
 
+// X += alpha_c P, then P = z + beta_c P from the cycle's result (with z set),
+// two entries per thread (k even); bound by HBM: at 96^3 x 32 it moves 1.0 GB
+// where the separate passes (Z written and read back, P read twice) moved
+// 1.6 GB.
+template <typename TZ>
+__global__ void __launch_bounds__(kBlock)
+k_bl_dirx(long long half, int k, const double* __restrict__ alpha, const double* __restrict__ beta,
+          const TZ* __restrict__ z, double* __restrict__ X, double* __restrict__ P) {
+  for (long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x; e < half;
+       e += (long long)gridDim.x * blockDim.x) {
+    const int c = (int)((2 * e) % k);
+    double2 p = reinterpret_cast<const double2*>(P)[e];
+    double2 x = reinterpret_cast<const double2*>(X)[e];
+    x.x += alpha[c] * p.x;
+    x.y += alpha[c + 1] * p.y;
+    reinterpret_cast<double2*>(X)[e] = x;
+    if (z) {
+      p.x = (double)z[2 * e] + beta[c] * p.x;
+      p.y = (double)z[2 * e + 1] + beta[c + 1] * p.y;
+      reinterpret_cast<double2*>(P)[e] = p;
+    }
+  }
+}
+
 template <typename TS, typename TD>
 __global__ void k_bl_convert(long long n, const TS* __restrict__ s, TD* __restrict__ d) {
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n;
@@ -551,18 +615,32 @@ int vec_grid(const void* f, int nrows, int tpr, int max_grid, int nb_cap = 0) {
 template <typename TA, typename T, int MODE>
 int spmm(cudaStream_t st, int max_grid, int nrows, int k, const int* rp, const int* ci, const TA* av,
          const T* X, const T* B, const T* dinv, T omega, T* Y, double* part = nullptr,
-         BlockShape sh = {}) {
+         BlockShape sh = {}, T* Y1 = nullptr, bool split = false) {
   constexpr int V = VecPiece<T>::V;
   if (k % V == 0 && aligned16(X) && aligned16(B) && aligned16(Y)) {
     const int t0 = tpr_for(k / V);
+    if (split) {  // one row per warp, the default lanes per group
+      switch (t0) {
+#define DR_SPMM_SPLIT(t)                                                                              \
+  case t: {                                                                                           \
+    auto kf = k_spmm_vec<TA, T, MODE, t, true>;                                                       \
+    kf<<<vec_grid((const void*)kf, nrows, 32, max_grid), kBlock, 0, st>>>(nrows, k, rp, ci, av, X, B, \
+                                                                          dinv, omega, Y, Y1, part);  \
+    break;                                                                                            \
+  }
+        DR_SPMM_SPLIT(1) DR_SPMM_SPLIT(2) DR_SPMM_SPLIT(4) DR_SPMM_SPLIT(8)
+#undef DR_SPMM_SPLIT
+      }
+      return 1;
+    }
     const int tpr = (sh.tpr >= t0 && sh.tpr <= 16 && (sh.tpr & (sh.tpr - 1)) == 0) ? sh.tpr : t0;
     int grid = 1;
     switch (tpr) {
 #define DR_SPMM_VEC(t)                                                                            \
   case t: {                                                                                       \
-    auto kf = k_spmm_vec<TA, T, MODE, t>;                                                         \
+    auto kf = k_spmm_vec<TA, T, MODE, t, false>;                                                  \
     grid = vec_grid((const void*)kf, nrows, t, max_grid, sh.nb);                                  \
-    kf<<<grid, kBlock, 0, st>>>(nrows, k, rp, ci, av, X, B, dinv, omega, Y, part);                \
+    kf<<<grid, kBlock, 0, st>>>(nrows, k, rp, ci, av, X, B, dinv, omega, Y, Y1, part);            \
     break;                                                                                        \
   }
       DR_SPMM_VEC(1) DR_SPMM_VEC(2) DR_SPMM_VEC(4) DR_SPMM_VEC(8) DR_SPMM_VEC(16)
@@ -570,7 +648,8 @@ int spmm(cudaStream_t st, int max_grid, int nrows, int k, const int* rp, const i
     }
     return grid;
   }
-  k_spmm<TA, T, MODE><<<warp_grid(nrows, max_grid), kBlock, 0, st>>>(nrows, k, rp, ci, av, X, B, dinv, omega, Y);
+  if constexpr (MODE != BM_JZRES)
+    k_spmm<TA, T, MODE><<<warp_grid(nrows, max_grid), kBlock, 0, st>>>(nrows, k, rp, ci, av, X, B, dinv, omega, Y);
   return 0;
 }
 
@@ -739,7 +818,14 @@ void DevHier::col_dots(int n, int k, const double* a, const double* b, double* d
 // One cycle of level l on k columns; returns where the result ended (X or
 // the level's partner buffer).
 template <typename T>
-T* DevHier::cycle_block(int l, T* X, const T* B, bool x_zero, const CycleOpts& o, int k) {
+T* DevHier::cycle_block(int l, T* X, const T* B, bool x_zero, const CycleOpts& o, int k, bool x1_ready) {
+  // rows of this matrix are split over a warp's groups: long rows, fewer warps
+  // than 32 per SM without the split, in a hierarchy that is not summed in
+  // the reference's order anyway
+  const bool vec = k % 4 == 0 && aligned16(B);
+  auto split = [&](const DevMat& M) {
+    return vec && any_tree_ && M.maxlen > 64 && (long long)M.n * tpr_for(k / 4) <= 32LL * 32 * nsm_;
+  };
   DevLevel& L = L_[l];
   BlockVecs<T>& V = bvecs<T>(l);
   const DevMat& A = L.A;
@@ -751,32 +837,46 @@ T* DevHier::cycle_block(int l, T* X, const T* B, bool x_zero, const CycleOpts& o
   T* t = (X == V.x) ? V.t : V.x;
   const BlockShape sj = shape_of(A.rp, BM_JACOBI, sizeof(T), k);
   int pre = o.pre;
+  bool have_r = false;
   if (x_zero) {
-    note_launch();
-    if (pre >= 1) {
+    if (x1_ready) {  // the restriction wrote the first Jacobi step
+      --pre;
+    } else if (pre == 1 && vec) {
+      note_launch();
+      spmm<T, T, BM_JZRES>(st_, max_grid_, n, k, A.rp, A.ci, av, B, B, dinv, om, V.r, nullptr,
+                           shape_of(A.rp, BM_RESID, sizeof(T), k), x, split(A));
+      --pre;
+      have_r = true;
+    } else if (pre >= 1) {
+      note_launch();
       k_bl_jz<T><<<grid_for((long long)n * k, max_grid_), kBlock, 0, st_>>>(n, k, B, dinv, om, x);
       --pre;
     } else {
+      note_launch();
       k_bl_fill<T><<<grid_for((long long)n * k, max_grid_), kBlock, 0, st_>>>((long long)n * k, x);
     }
   }
   for (int s = 0; s < pre; ++s) {
     note_launch();
-    spmm<T, T, BM_JACOBI>(st_, max_grid_, n, k, A.rp, A.ci, av, x, B, dinv, om, t, nullptr, sj);
+    spmm<T, T, BM_JACOBI>(st_, max_grid_, n, k, A.rp, A.ci, av, x, B, dinv, om, t, nullptr, sj, (T*)nullptr, split(A));
     std::swap(x, t);
   }
-  note_launch();
-  spmm<T, T, BM_RESID>(st_, max_grid_, n, k, A.rp, A.ci, av, x, B, nullptr, T(0), V.r, nullptr,
-                       shape_of(A.rp, BM_RESID, sizeof(T), k));
+  if (!have_r) {
+    note_launch();
+    spmm<T, T, BM_RESID>(st_, max_grid_, n, k, A.rp, A.ci, av, x, B, nullptr, T(0), V.r, nullptr,
+                         shape_of(A.rp, BM_RESID, sizeof(T), k), (T*)nullptr, split(A));
+  }
   const bool last = (l + 1 == nlevels());
   T* bc = last ? (sizeof(T) == 8 ? (T*)bcb64_ : (T*)bcb32_) : bvecs<T>(l + 1).b;
   const DevMat& R = L.R;
   note_launch();
-  spmm<T, T, BM_STORE>(st_, max_grid_, R.n, k, R.rp, R.ci, mval<T>(R), V.r, nullptr, nullptr, T(0), bc, nullptr,
-                       shape_of(R.rp, BM_STORE, sizeof(T), k));
+  const bool x1n = !last && vec && o.pre >= 1;
+  spmm<T, T, BM_STORE>(st_, max_grid_, R.n, k, R.rp, R.ci, mval<T>(R), V.r, nullptr,
+                       x1n ? invd<T>(L_[l + 1]) : nullptr, x1n ? (T)L_[l + 1].omega : T(0), bc, nullptr,
+                       shape_of(R.rp, BM_STORE, sizeof(T), k), x1n ? bvecs<T>(l + 1).x : nullptr, split(R));
   T* xc;
   if (!last) {
-    xc = cycle_block<T>(l + 1, bvecs<T>(l + 1).x, bc, true, o, k);
+    xc = cycle_block<T>(l + 1, bvecs<T>(l + 1).x, bc, true, o, k, x1n);
     if (o.w) xc = cycle_block<T>(l + 1, xc, bc, false, o, k);
   } else {
     xc = sizeof(T) == 8 ? (T*)bcx64_ : (T*)bcx32_;
@@ -807,7 +907,7 @@ T* DevHier::cycle_block(int l, T* X, const T* B, bool x_zero, const CycleOpts& o
     // correction and the first post-smoothing step in one pass over Q (see
     // EpCorrectJacobi; V.r holds B - A x from the way down)
     spmm<T, T, BM_CORRECT>(st_, max_grid_, L.AP.n, k, L.AP.rp, L.AP.ci, qval<T>(L), xc, V.r, dinv, om, x,
-                           nullptr, shape_of(L.AP.rp, BM_CORRECT, sizeof(T), k));
+                           nullptr, shape_of(L.AP.rp, BM_CORRECT, sizeof(T), k), (T*)nullptr, split(L.AP));
     post0 = 1;
   } else {
     spmm<T, T, BM_ADDTO>(st_, max_grid_, P.n, k, P.rp, P.ci, mval<T>(P), xc, nullptr, nullptr, T(0), x, nullptr,
@@ -815,15 +915,15 @@ T* DevHier::cycle_block(int l, T* X, const T* B, bool x_zero, const CycleOpts& o
   }
   for (int s = post0; s < o.post; ++s) {
     note_launch();
-    spmm<T, T, BM_JACOBI>(st_, max_grid_, n, k, A.rp, A.ci, av, x, B, dinv, om, t, nullptr, sj);
+    spmm<T, T, BM_JACOBI>(st_, max_grid_, n, k, A.rp, A.ci, av, x, B, dinv, om, t, nullptr, sj, (T*)nullptr, split(A));
     std::swap(x, t);
   }
   DR_CK(cudaGetLastError());
   return x;
 }
 
-template float* DevHier::cycle_block<float>(int, float*, const float*, bool, const CycleOpts&, int);
-template double* DevHier::cycle_block<double>(int, double*, const double*, bool, const CycleOpts&, int);
+template float* DevHier::cycle_block<float>(int, float*, const float*, bool, const CycleOpts&, int, bool);
+template double* DevHier::cycle_block<double>(int, double*, const double*, bool, const CycleOpts&, int, bool);
 
 int DevHier::pcg_block(double* X, const double* B, int k, const CycleOpts& o, double tol, int maxiter,
                        bool mixed, int* iters, double* relres, int verbose) {
@@ -859,14 +959,14 @@ int DevHier::pcg_block(double* X, const double* B, int k, const CycleOpts& o, do
     note_launch();
     k_bl_dot_final<<<1, 1024, 0, st_>>>(nblocks, k, bpart_, dst);
   };
-  auto update = [&](bool r32) {  // X += alpha P, R -= alpha Q, r.r -> dv[1]
+  auto update = [&](bool r32) {  // R -= alpha Q, r.r -> dv[1]; X += alpha P here only when not fused
     note_launch();
     if (fused) {
       float* r32p = r32 ? R32 : nullptr;
       switch (tpr2) {
 #define DR_UPD(t)                                                                             \
   case t:                                                                                     \
-    k_bl_update_vec<t><<<g2, kBlock, 0, st_>>>(n, k, dv + 4 * 32, X, R, P, Q, r32p, bpart_); \
+    k_bl_update_vec<t><<<g2, kBlock, 0, st_>>>(n, k, dv + 4 * 32, R, Q, r32p, bpart_);       \
     break;
         DR_UPD(1) DR_UPD(2) DR_UPD(4) DR_UPD(8) DR_UPD(16)
 #undef DR_UPD
@@ -878,7 +978,7 @@ int DevHier::pcg_block(double* X, const double* B, int k, const CycleOpts& o, do
     }
   };
   bool r32_ready = false;  // R32 already holds (float) R
-  auto take_z = [&](const auto* z) {  // Z = z, r.z -> dv[2]
+  auto take_z = [&](const auto* z, double* Z) {  // r.z -> dv[2], and Z = z when Z is set
     using TZ = std::remove_const_t<std::remove_pointer_t<decltype(z)>>;
     note_launch();
     if (fused) {
@@ -896,18 +996,32 @@ int DevHier::pcg_block(double* X, const double* B, int k, const CycleOpts& o, do
       col_dots(n, k, R, Z, dv + 2 * 32);
     }
   };
-  auto precond = [&]() {  // Z = M R, then r.z -> dv[2]
+  const void* zcur = nullptr;  // where the last cycle ended
+  auto precond = [&](double* Zout) {  // z = M R, then r.z -> dv[2], and Zout = z when set
     if (mixed) {
       if (!r32_ready) {
         note_launch();
         k_bl_convert<double, float><<<vgrid, kBlock, 0, st_>>>(m, R, R32);
       }
       const float* z = cycle_block<float>(0, bvecs<float>(0).x, R32, true, o, k);
-      take_z(z);
+      zcur = z;
+      take_z(z, Zout);
     } else {
       const double* z = cycle_block<double>(0, bvecs<double>(0).x, R, true, o, k);
-      take_z(z);
+      zcur = z;
+      take_z(z, Zout);
     }
+  };
+  // X += alpha P and, unless `last`, P = z + beta P with the cycle's z
+  auto dirx = [&](bool last) {
+    note_launch();
+    const long long half = m / 2;
+    const int g = grid_for(half, max_grid_);
+    const double *al = dv + 4 * 32, *be = dv + 5 * 32;
+    if (mixed)
+      k_bl_dirx<float><<<g, kBlock, 0, st_>>>(half, k, al, be, last ? nullptr : (const float*)zcur, X, P);
+    else
+      k_bl_dirx<double><<<g, kBlock, 0, st_>>>(half, k, al, be, last ? nullptr : (const double*)zcur, X, P);
   };
   note_launch();
   spmm<double, double, BM_RESID>(st_, max_grid_, n, k, A.rp, A.ci, A.v, X, B, nullptr, 0.0, R);
@@ -924,9 +1038,8 @@ int DevHier::pcg_block(double* X, const double* B, int k, const CycleOpts& o, do
     active[c] = bb[c] > 0.0 && std::sqrt(rr[c] / bb[c]) >= tol;
     nact += active[c];
   }
-  precond();
+  precond(P);  // the first direction
   fetch(2);
-  DR_CK(cudaMemcpyAsync(P, Z, (size_t)m * sizeof(double), cudaMemcpyDeviceToDevice, st_));
   DR_CK(cudaStreamSynchronize(st_));
   std::vector<double> rz(hv + 64, hv + 64 + k);
   int it = 0;
@@ -954,8 +1067,11 @@ int DevHier::pcg_block(double* X, const double* B, int k, const CycleOpts& o, do
         }
       }
     if (verbose >= 2) std::printf("  block PCG iter %4d: %d of %d columns active\n", it, nact, k);
-    if (nact == 0) break;
-    precond();
+    if (nact == 0) {
+      if (fused) dirx(true);
+      break;
+    }
+    precond(fused ? nullptr : Z);
     fetch(2);
     DR_CK(cudaStreamSynchronize(st_));
     for (int c = 0; c < k; ++c) {
@@ -964,8 +1080,12 @@ int DevHier::pcg_block(double* X, const double* B, int k, const CycleOpts& o, do
       rz[c] = rzn;
     }
     DR_CK(cudaMemcpyAsync(dv + 5 * 32, hv + 5 * 32, k * sizeof(double), cudaMemcpyHostToDevice, st_));
-    note_launch();
-    k_bl_dir<<<vgrid, kBlock, 0, st_>>>(n, k, dv + 5 * 32, Z, P);
+    if (fused) {
+      dirx(false);
+    } else {
+      note_launch();
+      k_bl_dir<<<vgrid, kBlock, 0, st_>>>(n, k, dv + 5 * 32, Z, P);
+    }
   }
   // true residuals of the result
   note_launch();

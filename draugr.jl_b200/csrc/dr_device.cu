@@ -496,9 +496,8 @@ DevHier::DevHier(const HostHierarchy& H, int device, const BatchLayout* batch) {
     if (!batch) {
       // the coarsest inverse, for hierarchies whose cycle is not bit-exact
       // anyway (some level sums its rows in a tree)
-      bool any_tree = false;
-      for (int l = 0; l < nl; ++l) any_tree = any_tree || !L_[l].A.form.ordered;
-      cinv_ok_ = any_tree && nc_ >= 1 && nc_ <= kern::kInvMax;
+      for (int l = 0; l < nl; ++l) any_tree_ = any_tree_ || !L_[l].A.form.ordered;
+      cinv_ok_ = any_tree_ && nc_ >= 1 && nc_ <= kern::kInvMax;
       if (cinv_ok_) build_cinv();
     }
     if (batch) tail_ = nl;  // no shared-memory tail: every level runs as its own launches

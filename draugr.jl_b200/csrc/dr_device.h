@@ -383,7 +383,7 @@ class DevHier {
   template <typename T>
   BlockVecs<T>& bvecs(int l);
   template <typename T>
-  T* cycle_block(int l, T* X, const T* B, bool x_zero, const CycleOpts& o, int k);
+  T* cycle_block(int l, T* X, const T* B, bool x_zero, const CycleOpts& o, int k, bool x1_ready = false);
   void col_dots(int n, int k, const double* a, const double* b, double* dst_dev);
   // transposed hierarchy (adjoint solves)
   bool at_built_ = false;
@@ -472,6 +472,7 @@ class DevHier {
   // and the block cycle apply instead of the substitutions when the cycle
   // is not bit-exact anyway (some level sums its rows in a tree)
   double* cinv_ = nullptr;
+  bool any_tree_ = false;  // some level sums its rows in a tree
   bool cinv_ok_ = false;   // cinv_ is kept (such a hierarchy, n_c <= 64)
   bool tail_inv_ = false;  // the tail applies it
   void build_cinv();
