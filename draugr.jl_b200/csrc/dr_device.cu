@@ -1832,7 +1832,8 @@ void DevHier::batch_coarse(int l, const T* b, T* x) {
   counted();
   const size_t wsm = (size_t)(c.maxn + (size_t)c.maxn * c.maxn) * sizeof(double);
   if (c.inv) {  // one block per system, x = A^-1 b
-    k_inv_apply_batch<T><<<c.nblk, kern::kInvMax, 0, st_>>>(c.off, c.nb, c.luoff, binv_, b, x);
+    launch_dependent(k_inv_apply_batch<T>, c.nblk, kern::kInvMax, 0, st_, (const int*)c.off, (const int*)c.nb,
+                     (const long long*)c.luoff, (const double*)binv_, b, x);
   } else if (wsm <= 48 * 1024) {  // one warp per system, its factors staged in shared memory
     k_lu_solve_batch_warp<T><<<c.nblk, 32, wsm, st_>>>(c.off, c.nb, c.luoff, c.poff, blu_, bpiv_, b, x, c.maxn);
   } else {
