@@ -1554,11 +1554,15 @@ k_lu_solve_t_warp(int n, const double* __restrict__ lu_g, const int* __restrict_
 
 // In-place unblocked LU with partial pivoting (dgetf2 order) of a
 // column-major n x n matrix in one block.  info = 0 or the 1-based index of
-// the first zero pivot (factorisation stops there).
+// the first zero pivot (factorisation stops there).  Whether the pivot is
+// zero is decided once, with the search, and published beside its row: the
+// interchange begins right after, so a thread that read the matrix again could
+// see the old diagonal entry.
 __global__ void k_lu_factor(int n, double* __restrict__ a, int* __restrict__ piv, int* info) {
   __shared__ double sv[1024];
   __shared__ int si[1024];
   __shared__ int sp;
+  __shared__ bool zero;
   if (threadIdx.x == 0) *info = 0;
   for (int j = 0; j < n; ++j) {
     // pivot search: first index of the maximum magnitude in column j
@@ -1585,10 +1589,11 @@ __global__ void k_lu_factor(int n, double* __restrict__ a, int* __restrict__ piv
     if (threadIdx.x == 0) {
       sp = si[0];
       piv[j] = sp;
+      zero = sv[0] == 0.0;
     }
     __syncthreads();
     const int p = sp;
-    if (a[(size_t)j * n + p] == 0.0) {
+    if (zero) {
       if (threadIdx.x == 0) *info = j + 1;
       return;
     }
@@ -1625,6 +1630,7 @@ __global__ void __launch_bounds__(kLuThreads)
 k_lu_factor_small(int n, double* __restrict__ a, int* __restrict__ piv, int* info) {
   __shared__ double s[kInvMax * (kInvMax + 1)];
   __shared__ int sp;
+  __shared__ bool zero;
   constexpr int ld = kInvMax + 1;  // a_ij at s[j * ld + i]
   for (int t = threadIdx.x; t < n * n; t += kLuThreads) s[t / n * ld + t % n] = a[t];
   if (threadIdx.x == 0) *info = 0;
@@ -1648,11 +1654,12 @@ k_lu_factor_small(int n, double* __restrict__ a, int* __restrict__ piv, int* inf
         // every comparison fails on a column of NaNs: keep the row, as dgetf2 does
         sp = bi < n ? bi : j;
         piv[j] = sp;
+        zero = best == 0.0;
       }
     }
     __syncthreads();
     const int p = sp;
-    if (s[j * ld + p] == 0.0) {
+    if (zero) {
       if (threadIdx.x == 0) *info = j + 1;
       break;
     }

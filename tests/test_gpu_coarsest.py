@@ -21,9 +21,22 @@ def dense_system(n, seed):
     return sp.csr_matrix(A)
 
 
-@pytest.mark.parametrize("n", [1, 2, 31, 32, 33, 48, 63, 64, 65])
-def test_factors_after_resetup(n):
-    A = dense_system(n, n)
+def zero_diagonal_system(n, seed):
+    """Diagonally dominant rows dealt in cyclic order: every diagonal entry is
+    exactly zero, and the first n - 1 columns need an interchange."""
+    rng = np.random.default_rng(seed)
+    A = rng.uniform(-1, 1, (n, n)) + 2 * n * np.eye(n)
+    A = np.roll(A, 1, axis=0)
+    A[np.arange(n), np.arange(n)] = 0.0
+    return sp.csr_matrix(A)
+
+
+@pytest.mark.parametrize("system", [dense_system, zero_diagonal_system])
+@pytest.mark.parametrize("n", [1, 2, 31, 32, 33, 48, 63, 64, 65, 90])
+def test_factors_after_resetup(n, system):
+    if n == 1:
+        system = dense_system
+    A = system(n, n)
     cfg = draugr.AMGConfig(coarsening=draugr.AggregationCoarsening(0.25), smoother=draugr.JacobiSmootherType(),
                            max_coarse_size=100)
     h = draugr.amg_setup(A, cfg)  # n <= 100: the coarsest system alone
