@@ -1587,7 +1587,8 @@ __global__ void k_lu_factor(int n, double* __restrict__ a, int* __restrict__ piv
       __syncthreads();
     }
     if (threadIdx.x == 0) {
-      sp = si[0];
+      // every comparison fails on a column of NaNs: keep the row
+      sp = si[0] < n ? si[0] : j;
       piv[j] = sp;
       zero = sv[0] == 0.0;
     }
@@ -1651,7 +1652,7 @@ k_lu_factor_small(int n, double* __restrict__ a, int* __restrict__ piv, int* inf
         if (v2 > best || (v2 == best && i2 < bi)) { best = v2; bi = i2; }
       }
       if (threadIdx.x == 0) {
-        // every comparison fails on a column of NaNs: keep the row, as dgetf2 does
+        // every comparison fails on a column of NaNs: keep the row
         sp = bi < n ? bi : j;
         piv[j] = sp;
         zero = best == 0.0;

@@ -49,6 +49,24 @@ def test_factors_after_resetup(n, system):
     assert np.array_equal(h.export(-1, "C_lu"), lu)
 
 
+@pytest.mark.parametrize("n", [8, 64, 65, 72])
+def test_factors_of_nan_values_keep_pivots_in_range(n):
+    """A resetup with NaN coefficients leaves pivots that the substitutions
+    can index with, and the next resetup recovers."""
+    A = dense_system(n, n)
+    cfg = draugr.AMGConfig(coarsening=draugr.AggregationCoarsening(0.25), smoother=draugr.JacobiSmootherType(),
+                           max_coarse_size=100)
+    h = draugr.amg_setup(A, cfg)
+    lu, piv = h.export(-1, "C_lu"), h.export(-1, "C_piv")
+    B = A.copy()
+    B.data = np.full_like(B.data, np.nan)
+    draugr.amg_resetup(h, B, cfg)
+    assert np.array_equal(h.export(-1, "C_piv"), np.arange(n))
+    draugr.amg_resetup(h, A, cfg)
+    assert np.array_equal(h.export(-1, "C_piv"), piv)
+    assert np.array_equal(h.export(-1, "C_lu"), lu)
+
+
 @pytest.mark.parametrize("A", [problems.poisson1d(1000), problems.anisotropic_27pt(11),
                                sp.csr_matrix(problems.poisson1d(300) + sp.eye(300) * 0 +
                                              sp.csr_matrix((np.ones(300), (np.zeros(300, int), np.arange(300))),
