@@ -1577,10 +1577,10 @@ int DevHier::bicgstab(double* x, const double* b, const CycleOpts& o, double tol
   };
   int it = 0;
   if (rel >= tol && maxiter > 0) {
-    iteration(0);
+    if (rho1 != 0.0) iteration(0);
     while (true) {
       ++it;
-      if (rho1 == 0.0) break;  // breakdown: r orthogonal to the shadow residual
+      if (rho1 == 0.0) break;  // breakdown: r orthogonal to the shadow residual, or no residual left
       if (it < maxiter) iteration(it & 1);
       DR_CK(cudaEventSynchronize(ev_[(it - 1) & 1]));
       const double* h = bi_host_ + ((it - 1) & 1) * BS_N;

@@ -55,6 +55,20 @@ def test_bicgstab_iterates(steps):
 
 
 @pytest.mark.parametrize("precision", ["fp64", "mixed"])
+@pytest.mark.parametrize("transpose", [False, True])
+def test_bicgstab_from_the_solution(transpose, precision):
+    """No residual at the start and a tolerance of zero: the solve ends on the
+    breakdown test and leaves x as it was."""
+    A = problems.poisson2d(12)
+    cfg = draugr.hypre_default_config(smoother=draugr.L1JacobiSmootherType())
+    h = draugr.amg_setup(A, cfg)
+    xs = np.random.default_rng(0).integers(-4, 5, A.shape[0]).astype(float)  # whole numbers: b is exact
+    x, it, rel = draugr.bicgstab(xs.copy(), A @ xs, h, cfg, tol=0.0, maxiter=5, transpose=transpose,
+                                 precision=precision)
+    assert np.array_equal(x, xs) and rel == 0.0 and it == 1
+
+
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
 @pytest.mark.parametrize("restart,maxiter", [(1, 3), (3, 3), (3, 7), (30, 4)])
 def test_fgmres_stops_where_asked(restart, maxiter, precision):
     A, cfg, h, b = system()
