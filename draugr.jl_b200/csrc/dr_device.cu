@@ -70,9 +70,10 @@ static int* err_flag() {
   return p;
 }
 
-// Polls a row kernel makes on a tile's copy before it gives up.  Only the
-// test hook draugr_b200_set_tile_wait_limit lowers it (0 makes every row
-// kernel give up at once and report the timeout).
+// Polls a row kernel makes on a tile's copy, and a Gauss-Seidel cluster on a
+// colour's values, before it gives up.  Only the test hook
+// draugr_b200_set_tile_wait_limit lowers it (0 makes every such kernel give
+// up at once and report the timeout).
 static std::atomic<int> g_tile_wait_limit{kern::kWaitLimit};
 static int tile_wait_limit() { return g_tile_wait_limit.load(std::memory_order_relaxed); }
 void set_tile_wait_limit(int polls) { g_tile_wait_limit.store(polls < 0 ? kern::kWaitLimit : polls); }
@@ -575,7 +576,7 @@ DevHier::~DevHier() {
   if (own_stream_ && own_st_) cudaStreamDestroy(own_st_);
 }
 
-// Raise if a row kernel reported a bounded wait that gave up (the flag is
+// Raise if a kernel reported a bounded wait that gave up (the flag is
 // cleared so the hierarchy stays usable).
 static void check_kernel_flag(cudaStream_t st, double* pinned) {
   volatile int* e = reinterpret_cast<int*>(pinned + SC_N);  // after the host mirror of the scalars
@@ -585,7 +586,7 @@ static void check_kernel_flag(cudaStream_t st, double* pinned) {
   if (*e) {
     DR_CK(cudaMemsetAsync(flag, 0, sizeof(int), st));
     DR_CK(cudaStreamSynchronize(st));
-    fail("a row kernel timed out waiting for its tile copy (results discarded)");
+    fail("a kernel timed out waiting for its copies (results discarded)");
   }
 }
 
@@ -1064,7 +1065,7 @@ void DevHier::gs_sweeps(const DevLevel& L, const DevMat& A, const T* b, T* x, in
       counted();
       launch_cluster(lim.blocks, kc, lim.blocks, kern::kGsThreads, smem, st_, A.n, L.ncolors,
                      (const int*)L.color_offd, (const int4*)L.gs_meta, (const int*)A.ci, mval<T>(A), b, invd<T>(L),
-                     x, steps, 0, err_flag());
+                     x, steps, 0, err_flag(), tile_wait_limit());
       return;
     }
     for (int s = 0; s < steps; ++s)

@@ -154,12 +154,13 @@ __host__ __device__ constexpr size_t gs_cluster_smem(int n, long long colours) {
 // Sweeps over all colours of one level in one cluster (gridDim.x = cluster
 // size).  coff[0..ncolors]: first position of each colour in meta; x: the
 // iterate in global memory, read at the start (zero instead with x_zero)
-// and written at the end.
+// and written at the end.  wait_limit: polls of a colour's mbarrier before a
+// thread gives up and flags the error.
 template <int G, typename T>
 __global__ void __launch_bounds__(kGsThreads, 1)
 k_gs_cluster(int n, int ncolors, const int* __restrict__ coff, const int4* __restrict__ meta,
              const int* __restrict__ ci, const T* __restrict__ av, const T* __restrict__ b,
-             const T* __restrict__ invd, T* __restrict__ x, int steps, int x_zero, int* err) {
+             const T* __restrict__ invd, T* __restrict__ x, int steps, int x_zero, int* err, int wait_limit) {
   extern __shared__ __align__(16) unsigned char gs_smem[];
   T* const xs = reinterpret_cast<T*>(gs_smem);
   uint64_t* const bars = reinterpret_cast<uint64_t*>(gs_smem + gs_cluster_smem<T>(n, 0));
@@ -197,12 +198,17 @@ k_gs_cluster(int n, int ncolors, const int* __restrict__ coff, const int4* __res
   cluster_wait();
   const unsigned xs_addr = smem_u32(xs), bars_addr = smem_u32(bars);
   int waited = 0;
+  // A thread whose wait runs out reads no more of the iterate, but its rows
+  // are still sent (the results are discarded), so that every mbarrier's bytes
+  // arrive and no group is left short of a lane.
   bool ok = true;
-  for (int t = 0; t < total && ok; ++t) {
+  for (int t = 0; t < total; ++t) {
     const int phase = (t < mine ? 0 : t / mine * ncolors) + cur.m.w;
-    for (; waited < phase && ok; ++waited) ok = cluster_wait_bounded(bars + waited, kWaitLimit);
-    if (!ok) break;
-    T sum = cur.dot(lane, ci, av, xs);
+    while (waited < phase && ok) {
+      ok = cluster_wait_bounded(bars + waited, wait_limit);
+      waited += ok;
+    }
+    T sum = ok ? cur.dot(lane, ci, av, xs) : T(0);
 #pragma unroll
     for (int o = G >> 1; o > 0; o >>= 1) sum += __shfl_xor_sync(gmask, sum, o);
     const T xn = xs[cur.m.x] + cd * (cb - sum);
@@ -218,11 +224,18 @@ k_gs_cluster(int n, int ncolors, const int* __restrict__ coff, const int4* __res
       if (t + 2 < total) m1 = __ldg(meta + at(t + 2));
     }
   }
-  for (; waited < nphase && ok; ++waited) ok = cluster_wait_bounded(bars + waited, kWaitLimit);
-  if (!ok) atomicExch(err, 1);
+  // Every value sent to this block has arrived before it writes its part of x
+  // and leaves, also when a wait gave up on the way.
+  bool landed = true;
+  while (waited < nphase && landed) {
+    landed = cluster_wait_bounded(bars + waited, kWaitLimit);
+    waited += landed;
+  }
+  if (!ok || !landed) atomicExch(err, 1);
   __syncwarp();
-  cluster_arrive();  // no block leaves while another may still send to it
+  cluster_arrive();  // this block sends no more: the others may leave
   for (int i = (int)rank * kGsThreads + (int)threadIdx.x; i < n; i += (int)C * kGsThreads) x[i] = xs[i];
+  __syncwarp();
   cluster_wait();
 }
 

@@ -279,11 +279,12 @@ int32_t draugr_b200_set_stream(int32_t handle, void *stream);
 int64_t draugr_b200_kernel_launches(void);
 
 /* Test hook, no counterpart in the reference: the number of polls a row
- * kernel makes on a tile's copy (an mbarrier wait) before it gives up,
- * flags the timeout and returns; the entry point that launched it then
- * returns -1 with "timed out" in draugr_amg_last_error.  A negative value
- * restores the default (2^22).  0 makes every row kernel give up at once,
- * which is how the timeout path is tested without a stuck copy. */
+ * kernel makes on a tile's copy, or a Gauss-Seidel cluster on a colour's
+ * values (mbarrier waits), before it gives up, flags the timeout and
+ * returns; the entry point that launched it then returns -1 with "timed
+ * out" in draugr_amg_last_error.  A negative value restores the default
+ * (2^22).  0 makes every such kernel give up at once, which is how the
+ * timeout path is tested without a stuck copy. */
 void draugr_b200_set_tile_wait_limit(int32_t polls);
 
 #ifdef __cplusplus

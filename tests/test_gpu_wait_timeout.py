@@ -1,4 +1,5 @@
-"""The row kernel's bounded wait, made to run out without a stuck copy.
+"""The bounded waits of the row kernel and of the Gauss-Seidel cluster, made
+to run out without a stuck copy.
 
 Every row kernel (k_tile_rows) waits on an mbarrier for the bulk copy of
 each tile.  A wait that gives up must not read the stage: the block flags
@@ -60,4 +61,28 @@ def test_wait_that_runs_out_reports_an_error_and_the_device_stays_usable():
     O = oracle.OracleHierarchy(h)
     want = O.cycle(np.zeros(n), bh)
     assert np.linalg.norm(xc - want) / np.linalg.norm(want) < 1e-12
+    h.free()
+
+
+@pytest.mark.parametrize("A", [problems.poisson2d(20), problems.poisson2d(46, 44), problems.anisotropic_27pt(12)],
+                         ids=["2_colours", "2_colours_full", "8_colours"])
+@pytest.mark.parametrize("steps", [1, 3])
+@pytest.mark.parametrize("precision", [0, 1])
+def test_gauss_seidel_cluster_that_gives_up(A, steps, precision):
+    """A thread of k_gs_cluster whose wait for the earlier colours runs out
+    flags the error and still sends its rows, so every block's mbarriers
+    complete and the cluster leaves together; the next call is right again."""
+    lib = draugr.load()
+    h = draugr.amg_setup(A, draugr.AMGConfig(coarsening=draugr.AggregationCoarsening(0.25),
+                                             smoother=draugr.ColoredGaussSeidelType(), max_coarse_size=20))
+    rng = np.random.default_rng(5)
+    x, b = rng.uniform(-1, 1, A.shape[0]), rng.uniform(-1, 1, A.shape[0])
+    want = h.level_op(0, 2, x, b, steps=steps, precision=precision)
+    try:
+        lib.draugr_b200_set_tile_wait_limit(0)
+        with pytest.raises(draugr.DraugrError, match="timed out"):
+            h.level_op(0, 2, x, b, steps=steps, precision=precision)
+    finally:
+        lib.draugr_b200_set_tile_wait_limit(-1)
+    assert np.array_equal(h.level_op(0, 2, x, b, steps=steps, precision=precision), want)
     h.free()
