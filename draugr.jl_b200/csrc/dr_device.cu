@@ -1044,6 +1044,27 @@ void DevHier::refresh_fp32() {
 }
 
 // ------------------------------------------------------------ cycle pieces
+// Lanes per row of k_gs_color: the fewest that hold a row of 1.1 times the mean
+// length in their kGsBatch registers each.  A large level is bound by the
+// loads it issues, of which slots past a row's end are a part.  us per sweep
+// with 1, 2, 4, 8, 16, 32 lanes (FP64, - where not measured):
+//   10^6 rows of 5 entries (2 colours)     23   32   50   98    -    -
+//   10^6 rows of 7 entries (2 colours)     32   40   60  104  286    -
+//   262 k rows of 27 entries (8 colours)    -   37   26   42   67  108
+//   200 k rows of 41 entries (21 colours)   -    -   76   50   75  107
+//   27 k rows of 131 entries (58 colours)   -    -    -    -  174  143
+// A row longer than that walks its remainder 0.3 us a step, and a lane more
+// per row costs 10 ps a row, so the lanes double while the longest row's
+// remainder costs more than they do (100 k rows of 3 entries, three of 700:
+// 204 us with 1 lane, 26 with 16).
+static int gs_color_lanes(const DevMat& A) {
+  int G = 1;
+  while (G < 32 && 8.0 * G * A.n < 1.1 * A.nnz) G *= 2;
+  while (G < 32 && A.maxlen > 8 * G && A.maxlen * 30000.0 > (double)A.n * G * G) G *= 2;
+  return G;
+}
+static_assert(kern::kGsBatch == 8, "gs_color_lanes counts on 8 entries per lane");
+
 // `steps` coloured Gauss-Seidel sweeps on level L, in place: one launch of
 // one cluster when the iterate fits in a block's shared memory and a colour
 // holds, on average, no more rows than the cluster has row groups (one round
@@ -1055,7 +1076,7 @@ void DevHier::refresh_fp32() {
 template <typename T>
 void DevHier::gs_sweeps(const DevLevel& L, const DevMat& A, const T* b, T* x, int steps) {
   if (steps <= 0 || A.n <= 0) return;
-  auto run = [&](auto tag) {
+  auto cluster = [&](auto tag) {
     constexpr int G = decltype(tag)::value;
     auto kc = k_gs_cluster<G, T>;
     const ClusterLimits lim = cluster_limits(kc, kern::kGsThreads);
@@ -1066,8 +1087,13 @@ void DevHier::gs_sweeps(const DevLevel& L, const DevMat& A, const T* b, T* x, in
       launch_cluster(lim.blocks, kc, lim.blocks, kern::kGsThreads, smem, st_, A.n, L.ncolors,
                      (const int*)L.color_offd, (const int4*)L.gs_meta, (const int*)A.ci, mval<T>(A), b, invd<T>(L),
                      x, steps, 0, err_flag(), tile_wait_limit());
-      return;
+      return true;
     }
+    return false;
+  };
+  if (A.nnz >= 24LL * A.n ? cluster(std::integral_constant<int, 32>{}) : cluster(std::integral_constant<int, 8>{}))
+    return;
+  auto colours = [&](auto kf, int G) {
     for (int s = 0; s < steps; ++s)
       for (int c = 0; c < L.ncolors; ++c) {
         const int off = L.color_off[c];
@@ -1075,12 +1101,16 @@ void DevHier::gs_sweeps(const DevLevel& L, const DevMat& A, const T* b, T* x, in
         if (cnt == 0) continue;
         const int grid = (int)std::min<long long>(((long long)cnt * G + kBlock - 1) / kBlock, max_grid_);
         counted();
-        launch_dependent(k_gs_color<G, T>, grid, kBlock, 0, st_, cnt, (const int4*)(L.gs_meta + off),
-                         (const int*)A.ci, mval<T>(A), b, invd<T>(L), x);
+        launch_dependent(kf, grid, kBlock, 0, st_, cnt, (const int4*)(L.gs_meta + off), (const int*)A.ci,
+                         mval<T>(A), b, invd<T>(L), x);
       }
   };
-  if (A.nnz >= 24LL * A.n) run(std::integral_constant<int, 32>{});
-  else run(std::integral_constant<int, 8>{});
+  switch (gs_color_lanes(A)) {
+#define DR_GS_COLOR(g) \
+  case g: colours(k_gs_color<g, T>, g); break;
+    DR_GS_COLOR(1) DR_GS_COLOR(2) DR_GS_COLOR(4) DR_GS_COLOR(8) DR_GS_COLOR(16) DR_GS_COLOR(32)
+#undef DR_GS_COLOR
+  }
 }
 
 template <typename T>

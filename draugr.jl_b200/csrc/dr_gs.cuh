@@ -34,7 +34,7 @@
 //       iterate does not fit in shared memory or whose colours hold many
 //       rows; launched with programmatic stream serialization, the row's
 //       bounds and first entries loaded before the wait for the previous
-//       colour.
+//       colour; 1 to 32 lanes per row by its length (gs_color_lanes).
 //
 // Row update: x_i += invd_i·(b_i - A_i x)          (src/smoothers.jl:203-217)
 #pragma once
@@ -119,10 +119,12 @@ struct GsRow {
         }
       }
   }
-  // Σ a_ij x_j over this lane's entries
+  // Σ a_ij x_j over this lane's entries, in four interleaved sums (with one
+  // lane per row, a row's rounding errors are then those of a sum over four
+  // lanes)
   __device__ __forceinline__ T dot(int lane, const int* __restrict__ ci, const T* __restrict__ av,
                                    const T* x) const {
-    T sum = T(0);
+    T s[4] = {T(0), T(0), T(0), T(0)};
 #pragma unroll
     for (int h = 0; h < B; h += 8)
       if (m.y + h * G < m.z) {
@@ -131,10 +133,10 @@ struct GsRow {
         for (int j = 0; j < 8; ++j) xv[j] = x[c[h + j]];
 #pragma unroll
         for (int j = 0; j < 8; ++j)
-          if (m.y + lane + (h + j) * G < m.z) sum += v[h + j] * xv[j];
+          if (m.y + lane + (h + j) * G < m.z) s[j & 3] += v[h + j] * xv[j];
       }
-    for (int k = m.y + lane + B * G; k < m.z; k += G) sum += __ldg(av + k) * x[__ldg(ci + k)];
-    return sum;
+    for (int k = m.y + lane + B * G; k < m.z; k += G) s[0] += __ldg(av + k) * x[__ldg(ci + k)];
+    return (s[0] + s[1]) + (s[2] + s[3]);
   }
 };
 

@@ -33,6 +33,24 @@ def banded(n, width):
                     format="csr").sorted_indices()
 
 
+def nine_point(m):
+    """9-point stencil on m^2 nodes: 4 colours."""
+    t = sp.diags([np.ones(m - 1), np.ones(m), np.ones(m - 1)], [-1, 0, 1])
+    return sp.csr_matrix(9 * sp.eye(m * m) - sp.kron(t, t)).sorted_indices()
+
+
+def with_long_rows(A, nlong, length):
+    """Couple nlong rows, far from one another, to `length` columns each."""
+    n = A.shape[0]
+    rng = np.random.default_rng(6)
+    rows = np.repeat(np.arange(nlong) * (n // nlong), length)
+    cols = rng.choice(n, size=nlong * length, replace=False)
+    C = sp.csr_matrix((np.full(len(rows), -0.01), (rows, cols)), shape=A.shape)
+    C = sp.csr_matrix(C + C.T)
+    C.setdiag(0)
+    return sp.csr_matrix(A + C + sp.diags(np.asarray(-C.sum(1)).ravel())).sorted_indices()
+
+
 def sweeps(A, order, off, invd, x, b, steps):
     x = x.copy()
     for _ in range(steps):
@@ -72,3 +90,51 @@ def test_gs_sweeps(name, smoother):
             # a row's sum of `longest` products in another order, every sweep
             tol = 4 * eps * longest * steps
             assert np.linalg.norm(got - ref) <= tol * np.linalg.norm(ref), (steps, prec)
+
+
+# one launch per colour: matrix, lanes per row of its kernel
+COLOR_CASES = {
+    "poisson1d_3000": (lambda: problems.poisson1d(3000), 1),            # a partial last block
+    "poisson3d_20": (lambda: problems.poisson3d(20), 1),                # rows of 7 of the 8 a lane holds
+    "rows_9_of_1": (lambda: with_long_rows(problems.poisson1d(300001), 3, 6), 1),   # one entry left over
+    "nine_point_70": (lambda: nine_point(70), 2),
+    "fe27_22": (lambda: problems.anisotropic_27pt(22), 4),
+    "banded_41": (lambda: banded(12000, 20), 8),
+    "rows_700": (lambda: with_long_rows(problems.poisson1d(100000), 3, 700), 16),    # few long rows: more lanes
+    "banded_101": (lambda: banded(18000, 50), 16),
+    "banded_141": (lambda: banded(20000, 70), 32),
+    "rows_340": (lambda: with_long_rows(banded(20500, 70), 5, 200), 32),            # left over from 32 lanes
+}
+
+
+@pytest.mark.parametrize("name", list(COLOR_CASES))
+def test_colour_launches(name):
+    make, lanes = COLOR_CASES[name]
+    A = make()
+    n = A.shape[0]
+    h = draugr.amg_setup(A, draugr.AMGConfig(coarsening=draugr.AggregationCoarsening(0.25),
+                                             smoother=draugr.ColoredGaussSeidelType()))
+    order, off, invd = h.export(0, "color_order"), h.export(0, "color_offsets"), h.export(0, "invdiag")
+    longest = int(np.diff(A.indptr).max())
+    # the dispatch rule: 1.1 mean rows held by the lanes, more for few long rows
+    want = 1
+    while want < 32 and 8 * want * n < 1.1 * A.nnz:
+        want *= 2
+    while want < 32 and longest > 8 * want and longest * 30000 > n * want * want:
+        want *= 2
+    assert want == lanes
+    rng = np.random.default_rng(1)
+    x, b = rng.uniform(-1, 1, n), rng.uniform(-1, 1, n)
+    lib = draugr.load()
+    for prec, eps in ((0, 2.2e-16), (1, 1.2e-7)):
+        count = []
+        for steps in (1, 3):
+            ref = sweeps(A, order, off, invd, x, b, steps)
+            before = lib.draugr_b200_kernel_launches()
+            got = h.level_op(0, 2, x, b, steps=steps, precision=prec)
+            count.append(lib.draugr_b200_kernel_launches() - before)
+            # a row's sum of `longest` products in another order, every sweep
+            assert np.linalg.norm(got - ref) <= 4 * eps * longest * steps * np.linalg.norm(ref), (steps, prec)
+        if prec == 0:  # FP32's first call also converts the matrix
+            assert count[1] - count[0] == 2 * (len(off) - 1)
+    h.free()
