@@ -41,7 +41,11 @@ using namespace kern;
 // number of kernels captured in it on every launch).
 static std::atomic<long long> g_launches{0};
 long long kernel_launches() { return g_launches.load(); }
-static inline void counted() { g_launches.fetch_add(1, std::memory_order_relaxed); }
+static thread_local long long t_launches = 0;  // this thread's
+static inline void counted() {
+  g_launches.fetch_add(1, std::memory_order_relaxed);
+  ++t_launches;
+}
 void note_launch() { counted(); }
 
 // SM count of the device in use and a device flag the row kernels set when a
@@ -609,6 +613,26 @@ void DevHier::graphs_clear() {
   cycle_graphs_.clear();
 }
 
+// The graph (or first use) of a cycle on the vectors `in` and `out`, added if
+// it is new.
+DevHier::CycleGraph& DevHier::cycle_graph(int kind, const void* in, const void* out, const CycleOpts& o) {
+  const int key[6] = {kind, tr_ ? 1 : 0, o.pre, o.post, o.w ? 1 : 0, tile_wait_limit()};
+  for (CycleGraph& c : cycle_graphs_)
+    if (c.in == in && c.out == out && std::equal(key, key + 6, c.key)) return c;
+  if (cycle_graphs_.size() >= 16) {  // options keep changing: start over
+    DR_CK(cudaStreamSynchronize(st_));
+    for (CycleGraph& c : cycle_graphs_)
+      if (c.exec) cudaGraphExecDestroy(c.exec);
+    cycle_graphs_.clear();
+  }
+  cycle_graphs_.emplace_back();
+  CycleGraph& g = cycle_graphs_.back();
+  std::copy(key, key + 6, g.key);
+  g.in = in;
+  g.out = out;
+  return g;
+}
+
 // A cycle on the hierarchy's own vectors `in` and `out` as one graph launch:
 // `body` launches its kernels and returns where the result ended.  The
 // first use runs them as they are (a hierarchy used once pays no capture, and
@@ -625,23 +649,13 @@ void* DevHier::replay(int kind, const void* in, void* out, const CycleOpts& o, F
     ~Flag() { f = false; }
   } flag{in_replay_};
   in_replay_ = true;
-  const int key[6] = {kind, tr_ ? 1 : 0, o.pre, o.post, o.w ? 1 : 0, tile_wait_limit()};
-  CycleGraph* g = nullptr;
-  for (CycleGraph& c : cycle_graphs_)
-    if (c.in == in && c.out == out && std::equal(key, key + 6, c.key)) g = &c;
-  if (!g) {
-    if (cycle_graphs_.size() >= 16) {  // options keep changing: start over
-      DR_CK(cudaStreamSynchronize(st_));
-      for (CycleGraph& c : cycle_graphs_)
-        if (c.exec) cudaGraphExecDestroy(c.exec);
-      cycle_graphs_.clear();
-    }
-    cycle_graphs_.emplace_back();
-    g = &cycle_graphs_.back();
-    std::copy(key, key + 6, g->key);
-    g->in = in;
-    g->out = out;
-    return body();
+  CycleGraph* g = &cycle_graph(kind, in, out, o);
+  if (!g->used) {
+    const long long c0 = t_launches;
+    void* result = body();
+    g->launches = t_launches - c0;
+    g->used = true;  // only now: a first use that fails is tried again as it is
+    return result;
   }
   if (!g->exec) {
     cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
@@ -651,7 +665,7 @@ void* DevHier::replay(int kind, const void* in, void* out, const CycleOpts& o, F
       return body();  // a stream that cannot be captured
     }
     cudaGraph_t graph = nullptr;
-    const long long c0 = g_launches.load();
+    const long long c0 = t_launches;
     DR_CK(cudaStreamBeginCapture(st_, cudaStreamCaptureModeThreadLocal));
     try {
       g->result = body();
@@ -662,7 +676,7 @@ void* DevHier::replay(int kind, const void* in, void* out, const CycleOpts& o, F
       throw;
     }
     DR_CK(cudaStreamEndCapture(st_, &graph));
-    g->launches = g_launches.load() - c0;
+    g->launches = t_launches - c0;
     g_launches.fetch_sub(g->launches);
     const cudaError_t e = cudaGraphInstantiate(&g->exec, graph, 0);
     cudaGraphDestroy(graph);
@@ -671,6 +685,27 @@ void* DevHier::replay(int kind, const void* in, void* out, const CycleOpts& o, F
   DR_CK(cudaGraphLaunch(g->exec, st_));
   g_launches.fetch_add(g->launches);
   return g->result;
+}
+
+// A cycle on vectors other than the hierarchy's own needs copies around its
+// graph, which pay only where the launches they save take longer: runs `body`
+// (the same cycle, launched on the caller's vectors) and returns true unless
+// it has at least 26 kernels, and one for every 4000 rows.  us per amg_cycle
+// launched and as a graph with its three copies:
+//   2-D Jacobi, aggregation, 14 kernels: 65 k rows 61, 73; 160 k 79, 95
+//   3-D l1-Jacobi, 19-25 kernels: 33 k rows 81, 87; 141 k 109, 124
+//   2-D convection-diffusion, 38 kernels: 90 k rows 152, 154; 160 k 187, 198
+//   2-D Gauss-Seidel, 32-38 kernels: 4 k rows 166, 150; 10 k 175, 160
+//   3-D Gauss-Seidel, 176 kernels: 262 k rows 972, 938
+template <class F>
+bool DevHier::direct_cycle(int kind, const void* in, const void* out, const CycleOpts& o, F&& body) {
+  CycleGraph& g = cycle_graph(kind, in, out, o);
+  if (g.used && g.launches >= 26 && g.launches * 4000 >= n0_) return false;
+  const long long c0 = t_launches;
+  body();
+  g.launches = t_launches - c0;
+  g.used = true;
+  return true;
 }
 
 // ------------------------------------------------------------ typed accessors
@@ -1324,9 +1359,6 @@ T* DevHier::cycle_level(int l, T* x, const T* b, bool x_zero, const CycleOpts& o
   return x;
 }
 
-// Largest finest level whose amg_cycle runs as a graph.
-static constexpr int kCycleGraphRows = 300000;
-
 void DevHier::cycle(double* x, const double* b, const CycleOpts& o) {
   if (L_.empty()) {
     coarse_solve<double>(b, x);
@@ -1337,15 +1369,8 @@ void DevHier::cycle(double* x, const double* b, const CycleOpts& o) {
     if (xo != xv)
       DR_CK(cudaMemcpyAsync(xv, xo, (size_t)n0_ * sizeof(double), cudaMemcpyDeviceToDevice, st_));
   };
-  // The graph works on the hierarchy's own vectors: three copies of the
-  // caller's, worth it while launching the kernels one by one takes the host
-  // longer than they run (41^3, 69 k rows: 116 us with launches, 106 with
-  // the graph; 128^3: the kernels take 0.6 ms, the copies 25 us).
+  if (direct_cycle(0, bd_, xd_, o, [&]() { run(x, b); })) return;
   const size_t bytes = (size_t)n0_ * sizeof(double);
-  if (n0_ > kCycleGraphRows) {
-    run(x, b);
-    return;
-  }
   if (b != bd_) DR_CK(cudaMemcpyAsync(bd_, b, bytes, cudaMemcpyDeviceToDevice, st_));
   if (x != xd_) DR_CK(cudaMemcpyAsync(xd_, x, bytes, cudaMemcpyDeviceToDevice, st_));
   replay(0, bd_, xd_, o, [&]() -> void* {
@@ -1732,13 +1757,11 @@ int DevHier::fgmres(double* x, const double* b, const CycleOpts& o, double tol, 
       double* vj = V + (size_t)j * n;
       double* zj = Z + (size_t)j * n;
       if (mixed) precond32(vj, zj, o);
-      else {
+      else if (!direct_cycle(2, w, gm_z_, o, [&]() { precond64(vj, zj, o); })) {
         // through two vectors of its own, so that every step replays one graph
-        double* const fin = gm_w_;
-        double* const fout = gm_z_;
-        DR_CK(cudaMemcpyAsync(fin, vj, (size_t)n * sizeof(double), cudaMemcpyDeviceToDevice, st_));
-        precond64(fin, fout, o, true);
-        DR_CK(cudaMemcpyAsync(zj, fout, (size_t)n * sizeof(double), cudaMemcpyDeviceToDevice, st_));
+        DR_CK(cudaMemcpyAsync(w, vj, (size_t)n * sizeof(double), cudaMemcpyDeviceToDevice, st_));
+        precond64(w, gm_z_, o, true);
+        DR_CK(cudaMemcpyAsync(zj, gm_z_, (size_t)n * sizeof(double), cudaMemcpyDeviceToDevice, st_));
       }
       spmv(zj, w);
       // classical Gram-Schmidt, twice

@@ -509,14 +509,18 @@ class DevHier {
     int key[6] = {0, 0, 0, 0, 0, 0};  // kind, transposed, pre, post, W, wait limit
     const void* in = nullptr;
     const void* out = nullptr;
+    bool used = false;       // ran once without a graph
     void* result = nullptr;  // where the cycle ends
     cudaGraphExec_t exec = nullptr;
     long long launches = 0;  // kernels in it
   };
   std::vector<CycleGraph> cycle_graphs_;
   bool in_replay_ = false;
+  CycleGraph& cycle_graph(int kind, const void* in, const void* out, const CycleOpts& o);
   template <class F>
   void* replay(int kind, const void* in, void* out, const CycleOpts& o, F&& body);
+  template <class F>
+  bool direct_cycle(int kind, const void* in, const void* out, const CycleOpts& o, F&& body);
   cudaEvent_t ev_[2] = {nullptr, nullptr};
   // a second stream and two events, to fork and join a branch of a graph
   // capture (the PCG iterate update beside the preconditioner)
