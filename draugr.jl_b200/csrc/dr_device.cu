@@ -1491,8 +1491,14 @@ void DevHier::build_transpose() {
   DR_CK(cudaStreamSynchronize(st_));
 }
 
+// us with a thread per row, a warp per 16 rows and a warp per 4: 2 M rows of 7
+// entries 28, 59, 104; 278 k of 13 11, 13, 20; 262 k of 26 14, 13, 22; 69 k of 26
+// 5.1, 4.5, 7.0; 100 k of 81 20, 16, 24; 21 k of 19 8.4, 6.6, 5.9; 5.7 k of 18
+// 6.1, 4.8, 4.0.  A few long rows would be one thread's chain.
 void DevHier::l1_invdiag(const DevMat& M, double* invd) {
-  if (M.n >= 65536)
+  if (M.nnz < 14LL * M.n && M.maxlen <= 64)
+    k_l1_invdiag_short<<<grid1d(M.n, max_grid_), kBlock, 0, st_>>>(M.n, M.rp, M.v, invd);
+  else if (M.n >= 65536)
     k_l1_invdiag<16><<<grid1d(2LL * M.n, max_grid_), kBlock, 0, st_>>>(M.n, M.rp, M.v, invd);
   else
     k_l1_invdiag<4><<<grid1d(8LL * M.n, max_grid_), kBlock, 0, st_>>>(M.n, M.rp, M.v, invd);

@@ -1789,12 +1789,24 @@ __global__ void k_invdiag(int n, const int* __restrict__ rp, const int* __restri
   }
 }
 
-// src/smoothers.jl:816-827: 1/Σ|a_ij|, or 0 if the sum is <= eps.  A warp
-// takes kDiagRows rows (16, or 4 where there are few): it reads 32 entries of each at a time (coalesced, all
-// rows in flight) into shared memory, and one lane per row adds them in
-// column order.  HBM-bound on long matrices; one thread per row reading its
-// own entries took 265 us for the 7 levels of the 27-point 96^3 hierarchy,
-// 162 us this way.
+// src/smoothers.jl:816-827: 1/Σ|a_ij|, or 0 if the sum is <= eps, summed in
+// column order.  One thread per row, for short rows: neighbouring threads read
+// neighbouring entries.
+__global__ void __launch_bounds__(kBlock)
+k_l1_invdiag_short(int n, const int* __restrict__ rp, const double* __restrict__ v, double* __restrict__ invd) {
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+    const int e = __ldg(rp + i + 1);
+    double l1 = 0.0;
+    for (int k = __ldg(rp + i); k < e; ++k) l1 = __dadd_rn(l1, fabs(__ldg(v + k)));
+    invd[i] = l1 > 2.220446049250313e-16 ? __drcp_rn(l1) : 0.0;
+  }
+}
+
+// The same for long rows.  A warp takes kDiagRows rows (16, or 4 where there
+// are few): it reads 32 entries of each at a time (coalesced, all rows in
+// flight) into shared memory, and one lane per row adds them in column order.
+// HBM-bound on long matrices; one thread per row took 265 us for the 7 levels of
+// the 27-point 96^3 hierarchy, 162 us this way.
 template <int kDiagRows>
 __global__ void __launch_bounds__(kBlock)
 k_l1_invdiag(int n, const int* __restrict__ rp, const double* __restrict__ v, double* __restrict__ invd) {

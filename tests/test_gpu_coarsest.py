@@ -1,7 +1,7 @@
 """The coarsest level's kernels at the edges of their ranges: factors of 1 to
 64 unknowns (and 65, the general kernel) after a resetup against the setup's
 host factors bit for bit, the l1 diagonals of short, long and empty-tailed
-rows, and cycles through the explicit inverse against the oracle."""
+rows (a thread, or a warp per 4 or 16 rows), and cycles through the explicit inverse against the oracle."""
 
 import numpy as np
 import pytest
@@ -67,11 +67,11 @@ def test_factors_of_nan_values_keep_pivots_in_range(n):
     assert np.array_equal(h.export(-1, "C_lu"), lu)
 
 
-@pytest.mark.parametrize("A", [problems.poisson1d(1000), problems.anisotropic_27pt(11),
+@pytest.mark.parametrize("A", [problems.poisson1d(1000), problems.anisotropic_27pt(11), problems.anisotropic_27pt(41),
                                sp.csr_matrix(problems.poisson1d(300) + sp.eye(300) * 0 +
                                              sp.csr_matrix((np.ones(300), (np.zeros(300, int), np.arange(300))),
                                                            shape=(300, 300)))],
-                         ids=["3_per_row", "27_per_row", "one_full_row"])
+                         ids=["3_per_row", "27_per_row", "27_per_row_many", "one_full_row"])
 def test_l1_diagonal_after_resetup(A):
     A = sp.csr_matrix(A)
     A.sort_indices()
