@@ -628,7 +628,7 @@ int spmm(cudaStream_t st, int max_grid, int nrows, int k, const int* rp, const i
                                                                           dinv, omega, Y, Y1, part);  \
     break;                                                                                            \
   }
-        DR_SPMM_SPLIT(1) DR_SPMM_SPLIT(2) DR_SPMM_SPLIT(4) DR_SPMM_SPLIT(8)
+        DR_SPMM_SPLIT(2) DR_SPMM_SPLIT(4) DR_SPMM_SPLIT(8)
 #undef DR_SPMM_SPLIT
       }
       return 1;
@@ -819,12 +819,19 @@ void DevHier::col_dots(int n, int k, const double* a, const double* b, double* d
 // the level's partner buffer).
 template <typename T>
 T* DevHier::cycle_block(int l, T* X, const T* B, bool x_zero, const CycleOpts& o, int k, bool x1_ready) {
-  // rows of this matrix are split over a warp's groups: long rows, fewer warps
-  // than 32 per SM without the split, in a hierarchy that is not summed in
-  // the reference's order anyway
+  // Rows of this matrix are split over a warp's groups: long rows, groups of 2
+  // lanes or more (with 32 groups of one lane the shuffle tree costs more than
+  // the walk), few rows (fewer warps than 32 per SM without the split, at most
+  // 256 rows per SM), in a hierarchy that is not summed in the reference's order
+  // anyway.  us per iteration without and with the split, mixed: 60^3 k = 4 673
+  // and 866, 8 622 and 563, 16 623 and 471, 32 792 and 678; 80^3 k = 8 1036 and
+  // 1040 with level 2 (54 k rows of 71 entries) split too, 939 with the levels
+  // below it only; levels of shorter rows too, 44^3 k = 8 389 and 380, 338 by
+  // this rule.
   const bool vec = k % 4 == 0 && aligned16(B);
   auto split = [&](const DevMat& M) {
-    return vec && any_tree_ && M.maxlen > 64 && (long long)M.n * tpr_for(k / 4) <= 32LL * 32 * nsm_;
+    const int t = tpr_for(k / 4);
+    return vec && any_tree_ && M.maxlen > 64 && t >= 2 && (long long)M.n * std::max(t, 4) <= 32LL * 32 * nsm_;
   };
   DevLevel& L = L_[l];
   BlockVecs<T>& V = bvecs<T>(l);
