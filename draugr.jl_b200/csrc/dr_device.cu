@@ -690,17 +690,19 @@ void* DevHier::replay(int kind, const void* in, void* out, const CycleOpts& o, F
 // A cycle on vectors other than the hierarchy's own needs copies around its
 // graph, which pay only where the launches they save take longer: runs `body`
 // (the same cycle, launched on the caller's vectors) and returns true unless
-// it has at least 26 kernels, and one for every 4000 rows.  us per amg_cycle
+// it has at least 18 kernels and one for every 200 rows, where launching takes
+// longer than the kernels run, or 26 and one for every 4000.  us per amg_cycle
 // launched and as a graph with its three copies:
 //   2-D Jacobi, aggregation, 14 kernels: 65 k rows 61, 73; 160 k 79, 95
-//   3-D l1-Jacobi, 19-25 kernels: 33 k rows 81, 87; 141 k 109, 124
+//   3-D l1-Jacobi, 19-25 kernels: 14 k rows 72, 75; 33 k 81, 87; 141 k 109, 124
+//   2-D l1-Jacobi, 2 + 2 steps: 4 k rows 101, 92
 //   2-D convection-diffusion, 38 kernels: 90 k rows 152, 154; 160 k 187, 198
-//   2-D Gauss-Seidel, 32-38 kernels: 4 k rows 166, 150; 10 k 175, 160
+//   2-D Gauss-Seidel: 18 kernels, 1 k rows 119, 111; 38, 10 k 175, 160
 //   3-D Gauss-Seidel, 176 kernels: 262 k rows 972, 938
 template <class F>
 bool DevHier::direct_cycle(int kind, const void* in, const void* out, const CycleOpts& o, F&& body) {
   CycleGraph& g = cycle_graph(kind, in, out, o);
-  if (g.used && g.launches >= 26 && g.launches * 4000 >= n0_) return false;
+  if (g.used && g.launches >= 18 && g.launches * (g.launches >= 26 ? 4000 : 200) >= n0_) return false;
   const long long c0 = t_launches;
   body();
   g.launches = t_launches - c0;
@@ -1369,7 +1371,8 @@ void DevHier::cycle(double* x, const double* b, const CycleOpts& o) {
     if (xo != xv)
       DR_CK(cudaMemcpyAsync(xv, xo, (size_t)n0_ * sizeof(double), cudaMemcpyDeviceToDevice, st_));
   };
-  if (direct_cycle(0, bd_, xd_, o, [&]() { run(x, b); })) return;
+  const bool own = x == xd_ && b == bd_;  // the host-pointer call: nothing to copy
+  if (!own && direct_cycle(0, bd_, xd_, o, [&]() { run(x, b); })) return;
   const size_t bytes = (size_t)n0_ * sizeof(double);
   if (b != bd_) DR_CK(cudaMemcpyAsync(bd_, b, bytes, cudaMemcpyDeviceToDevice, st_));
   if (x != xd_) DR_CK(cudaMemcpyAsync(xd_, x, bytes, cudaMemcpyDeviceToDevice, st_));
