@@ -1123,7 +1123,7 @@ void DevHier::gs_sweeps(const DevLevel& L, const DevMat& A, const T* b, T* x, in
       counted();
       launch_cluster(lim.blocks, kc, lim.blocks, kern::kGsThreads, smem, st_, A.n, L.ncolors,
                      (const int*)L.color_offd, (const int4*)L.gs_meta, (const int*)A.ci, mval<T>(A), b, invd<T>(L),
-                     x, steps, 0, err_flag(), tile_wait_limit());
+                     x, steps, err_flag(), tile_wait_limit());
       return true;
     }
     return false;
@@ -1524,10 +1524,9 @@ void DevHier::refresh_transpose() {
   DR_CK(cudaGetLastError());
 }
 
-void DevHier::lin3(int n, double a, const double* x, double b, const double* y, double c, const double* z,
-                   double* out) {
+void DevHier::lin2(int n, double a, const double* x, double b, const double* y, double* out) {
   counted();
-  k_lin3<<<grid1d(n, max_grid_), kBlock, 0, st_>>>(n, a, x, b, y, c, z, out);
+  k_lin2<<<grid1d(n, max_grid_), kBlock, 0, st_>>>(n, a, x, b, y, out);
   DR_CK(cudaGetLastError());
 }
 
@@ -1591,7 +1590,7 @@ int DevHier::bicgstab(double* x, const double* b, const CycleOpts& o, double tol
   x = xd_;
   if (xout != x) DR_CK(cudaMemcpyAsync(x, xout, (size_t)n * sizeof(double), cudaMemcpyDeviceToDevice, st_));
   spmv(x, t);
-  lin3(n, 1.0, b, -1.0, t, 0.0, nullptr, r);  // r = b - A x
+  lin2(n, 1.0, b, -1.0, t, r);  // r = b - A x
   DR_CK(cudaMemcpyAsync(rh, r, (size_t)n * sizeof(double), cudaMemcpyDeviceToDevice, st_));
   double rho1 = dot_host(r, r, n);  // rh·r, and r·r
   double rel = std::sqrt(rho1) / bnorm;
@@ -1662,7 +1661,7 @@ int DevHier::bicgstab(double* x, const double* b, const CycleOpts& o, double tol
   }
   // true residual of the result
   spmv(x, t);
-  lin3(n, 1.0, b, -1.0, t, 0.0, nullptr, r);
+  lin2(n, 1.0, b, -1.0, t, r);
   rel = std::sqrt(dot_host(r, r, n)) / bnorm;
   if (xout != x) DR_CK(cudaMemcpyAsync(xout, x, (size_t)n * sizeof(double), cudaMemcpyDeviceToDevice, st_));
   check_kernel_flag(st_, hscal_);
@@ -1749,12 +1748,12 @@ int DevHier::fgmres(double* x, const double* b, const CycleOpts& o, double tol, 
   double rel = 1.0;
   while (true) {
     spmv(x, w);
-    lin3(n, 1.0, b, -1.0, w, 0.0, nullptr, w);  // w = b - A x
+    lin2(n, 1.0, b, -1.0, w, w);  // w = b - A x
     const double beta = std::sqrt(dot_host(w, w, n));
     rel = beta / bnorm;
     if (verbose >= 2) std::printf("  FGMRES restart at iter %4d: relative residual %.6e\n", it, rel);
     if (rel < tol || it >= maxiter) break;
-    lin3(n, 1.0 / beta, w, 0.0, w, 0.0, nullptr, V);  // V_0 = w / beta
+    lin2(n, 1.0 / beta, w, 0.0, w, V);  // V_0 = w / beta
     std::fill(g.begin(), g.end(), 0.0);
     g[0] = beta;
     int jn = 0;  // columns in this cycle
@@ -1859,7 +1858,7 @@ int DevHier::refine(double* x, const double* b, const CycleOpts& o, double tol, 
     x = ir_x_;
     while (true) {
       launch_rows(st_, max_grid_, A, A.v, XPlain<double>{x}, EpStore<double>{ir_r_});
-      lin3(n, 1.0, b, -1.0, ir_r_, 0.0, nullptr, ir_r_);  // r = b - A x (FP64)
+      lin2(n, 1.0, b, -1.0, ir_r_, ir_r_);  // r = b - A x (FP64)
       rel = std::sqrt(dot_host(ir_r_, ir_r_, n)) / bnorm;
       if (verbose >= 2) std::printf("  refinement step %3d: relative residual %.6e\n", outer, rel);
       if (rel < tol || outer >= max_outer) break;
@@ -1870,7 +1869,7 @@ int DevHier::refine(double* x, const double* b, const CycleOpts& o, double tol, 
       const int its = inner == 1 ? fgmres(ir_d_, ir_r_, o, inner_tol, inner_maxiter, 30, mixed, &rr, 0)
                                  : pcg(ir_d_, ir_r_, o, inner_tol, inner_maxiter, mixed, &rr, 0);
       total += its;
-      lin3(n, 1.0, x, 1.0, ir_d_, 0.0, nullptr, x);  // x += d
+      lin2(n, 1.0, x, 1.0, ir_d_, x);  // x += d
       if (its == 0) break;  // the inner solver made no progress
     }
     DR_CK(cudaMemcpyAsync(xout, ir_x_, (size_t)n * sizeof(double), cudaMemcpyDeviceToDevice, st_));

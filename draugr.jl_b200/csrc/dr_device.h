@@ -394,8 +394,7 @@ class DevHier {
   double* bk_[8] = {nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr};
   double *bi_scal_ = nullptr, *bi_part_ = nullptr;  // BiCGStab scalars and partial sums
   double* bi_host_ = nullptr;                      // pinned, two copies of the scalars
-  void lin3(int n, double a, const double* x, double b, const double* y, double c, const double* z,
-            double* out);
+  void lin2(int n, double a, const double* x, double b, const double* y, double* out);
   void precond64(const double* r, double* out, const CycleOpts& o, bool fixed = false);
   void precond32(const double* r, double* out, const CycleOpts& o);  // FP32 cycle, FP64 in and out
   // batch: layout, its device arrays per merged level (coarse blocks), the

@@ -155,14 +155,14 @@ __host__ __device__ constexpr size_t gs_cluster_smem(int n, long long colours) {
 
 // Sweeps over all colours of one level in one cluster (gridDim.x = cluster
 // size).  coff[0..ncolors]: first position of each colour in meta; x: the
-// iterate in global memory, read at the start (zero instead with x_zero)
-// and written at the end.  wait_limit: polls of a colour's mbarrier before a
-// thread gives up and flags the error.
+// iterate in global memory, read at the start and written at the end.
+// wait_limit: polls of a colour's mbarrier before a thread gives up and flags
+// the error.
 template <int G, typename T>
 __global__ void __launch_bounds__(kGsThreads, 1)
 k_gs_cluster(int n, int ncolors, const int* __restrict__ coff, const int4* __restrict__ meta,
              const int* __restrict__ ci, const T* __restrict__ av, const T* __restrict__ b,
-             const T* __restrict__ invd, T* __restrict__ x, int steps, int x_zero, int* err, int wait_limit) {
+             const T* __restrict__ invd, T* __restrict__ x, int steps, int* err, int wait_limit) {
   extern __shared__ __align__(16) unsigned char gs_smem[];
   T* const xs = reinterpret_cast<T*>(gs_smem);
   uint64_t* const bars = reinterpret_cast<uint64_t*>(gs_smem + gs_cluster_smem<T>(n, 0));
@@ -194,7 +194,7 @@ k_gs_cluster(int n, int ncolors, const int* __restrict__ coff, const int4* __res
     cb = __ldg(b + cur.m.x);
     cd = __ldg(invd + cur.m.x);
   }
-  for (int i = threadIdx.x; i < n; i += kGsThreads) xs[i] = x_zero ? T(0) : x[i];
+  for (int i = threadIdx.x; i < n; i += kGsThreads) xs[i] = x[i];
   __syncwarp();
   cluster_arrive();  // every block's copy and mbarriers are ready before any send
   cluster_wait();

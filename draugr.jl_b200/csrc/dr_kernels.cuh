@@ -797,14 +797,10 @@ __global__ void k_convert(long long n, const TS* __restrict__ s, TD* __restrict_
     d[i] = (TD)s[i];
 }
 
-// out = a x + b y + c z (out may be x, y or z; z may be null when c = 0)
-__global__ void k_lin3(int n, double a, const double* x, double b, const double* y, double c,
-                       const double* z, double* out) {
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-    double v = a * x[i] + b * y[i];
-    if (z) v += c * z[i];
-    out[i] = v;
-  }
+// out = a x + b y (out may be x or y)
+__global__ void k_lin2(int n, double a, const double* x, double b, const double* y, double* out) {
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
+    out[i] = a * x[i] + b * y[i];
 }
 
 // Gradient of a loss L(x), x = A^-1 b, with respect to the nonzeros of A,
