@@ -206,9 +206,11 @@ int32_t draugr_amg_resetup(int32_t handle, int32_t n, int32_t nnz, const int32_t
       DevHier& D = device_of(*H);
       double* tmp = nullptr;
       DR_CK(cudaMalloc(&tmp, std::max<size_t>(1, A.v.size()) * sizeof(double)));
-      cudaError_t e = cudaMemcpy(tmp, A.v.data(), A.v.size() * sizeof(double), cudaMemcpyHostToDevice);
       try {
-        DR_CK(e);
+        // on the hierarchy's stream, which resetup_values continues on: a plain
+        // cudaMemcpy may return with the last part still on the way, and that
+        // stream does not wait for the default one
+        DR_CK(cudaMemcpyAsync(tmp, A.v.data(), A.v.size() * sizeof(double), cudaMemcpyHostToDevice, D.stream()));
         D.resetup_values(tmp);
       } catch (...) {
         cudaFree(tmp);
@@ -785,8 +787,8 @@ int32_t draugr_b200_level_op(int32_t handle, int32_t lvl, int32_t op, int32_t pr
       DR_CK(cudaMalloc(&d1, std::max(1, n_in1) * sizeof(double)));
       DR_CK(cudaMalloc(&d2, std::max(1, n_in2) * sizeof(double)));
       DR_CK(cudaMalloc(&d3, std::max(1, n_out) * sizeof(double)));
-      DR_CK(cudaMemcpy(d1, in1, n_in1 * sizeof(double), cudaMemcpyHostToDevice));
-      if (n_in2) DR_CK(cudaMemcpy(d2, in2, n_in2 * sizeof(double), cudaMemcpyHostToDevice));
+      DR_CK(cudaMemcpyAsync(d1, in1, n_in1 * sizeof(double), cudaMemcpyHostToDevice, D.stream()));
+      if (n_in2) DR_CK(cudaMemcpyAsync(d2, in2, n_in2 * sizeof(double), cudaMemcpyHostToDevice, D.stream()));
       D.level_op(lvl, op, precision == 1, d1, d2, d3, steps);
       DR_CK(cudaMemcpy(out, d3, n_out * sizeof(double), cudaMemcpyDeviceToHost));
     } catch (...) {

@@ -69,6 +69,7 @@ static int* err_flag() {
   if (!p) {
     DR_CK(cudaMalloc(&p, sizeof(int)));
     DR_CK(cudaMemset(p, 0, sizeof(int)));
+    DR_CK(cudaStreamSynchronize(cudaStreamLegacy));  // the hierarchies' streams do not wait for it
     g_err_dev[dev].store(p, std::memory_order_release);
   }
   return p;
@@ -331,6 +332,19 @@ template <typename T>
 static void h2d(T* d, const std::vector<T>& h, cudaStream_t st) {
   if (!h.empty()) DR_CK(cudaMemcpyAsync(d, h.data(), h.size() * sizeof(T), cudaMemcpyHostToDevice, st));
 }
+// The same for a host array that does not outlive the call.  (A plain
+// cudaMemcpy from pageable memory may return with its last part still on the
+// way, on the default stream, which the hierarchy's streams do not wait for.)
+template <typename T>
+static void h2d_now(T* d, const std::vector<T>& h, cudaStream_t st) {
+  h2d(d, h, st);
+  DR_CK(cudaStreamSynchronize(st));
+}
+template <typename T>
+static void d2h_now(std::vector<T>& h, const T* d, cudaStream_t st) {
+  if (!h.empty()) DR_CK(cudaMemcpyAsync(h.data(), d, h.size() * sizeof(T), cudaMemcpyDeviceToHost, st));
+  DR_CK(cudaStreamSynchronize(st));
+}
 
 DevHier::DevHier(const HostHierarchy& H, int device, const BatchLayout* batch) {
   device_ = device;
@@ -377,8 +391,8 @@ DevHier::DevHier(const HostHierarchy& H, int device, const BatchLayout* batch) {
         }
         d.gs_meta = alloc<int4>(meta.size());
         d.color_offd = alloc<int>(h.color_off.size());
-        DR_CK(cudaMemcpy(d.gs_meta, meta.data(), meta.size() * sizeof(int4), cudaMemcpyHostToDevice));
-        DR_CK(cudaMemcpy(d.color_offd, h.color_off.data(), h.color_off.size() * sizeof(int), cudaMemcpyHostToDevice));
+        h2d(d.color_offd, h.color_off, st_);
+        h2d_now(d.gs_meta, meta, st_);
       }
       d.has_rap = h.has_rap_map;
       if (d.has_rap || !h.ap_rp.empty()) up_csr(d.AP, h.A.n, h.P.nc, h.ap_rp, h.ap_ci, nullptr);
@@ -550,9 +564,9 @@ void DevHier::upload_csr(DevMat& M, int n, int m, const std::vector<int>& rp, co
   M.tp = alloc<int>(tiles.size());
   M.ts = alloc<int>(tiles.size());
   M.tb = alloc<int>(base.size());
-  DR_CK(cudaMemcpy(M.tp, tiles.data(), tiles.size() * sizeof(int), cudaMemcpyHostToDevice));
-  DR_CK(cudaMemcpy(M.ts, tstart.data(), tstart.size() * sizeof(int), cudaMemcpyHostToDevice));
-  DR_CK(cudaMemcpy(M.tb, base.data(), base.size() * sizeof(int), cudaMemcpyHostToDevice));
+  h2d(M.tp, tiles, st_);
+  h2d(M.ts, tstart, st_);
+  h2d(M.tb, base, st_);
   // 16-bit column offsets from each tile's smallest column (8 padding
   // entries for the tile kernel's 16-byte-rounded copies)
   std::vector<uint16_t> off(ci.size() + 8, 0);
@@ -560,8 +574,8 @@ void DevHier::upload_csr(DevMat& M, int n, int m, const std::vector<int>& rp, co
     if (base[t] >= 0)
       for (int k = tstart[t]; k < tstart[t + 1]; ++k) off[k] = (uint16_t)(ci[k] - base[t]);
   M.cu = alloc<uint16_t>(off.size());
-  DR_CK(cudaMemcpy(M.cu, off.data(), off.size() * sizeof(uint16_t), cudaMemcpyHostToDevice));
-  }
+  h2d_now(M.cu, off, st_);
+}
 
 DevHier::~DevHier() {
   cudaSetDevice(device_);
@@ -866,7 +880,7 @@ void DevHier::build_tail() {
     total += tail_level_bytes<double>(d, flat_row);
     if (!jac || d.A.n > 4096 || total > kTailSmem) break;
     std::vector<int> rp(d.A.n + 1);
-    DR_CK(cudaMemcpy(rp.data(), d.A.rp, rp.size() * sizeof(int), cudaMemcpyDeviceToHost));
+    d2h_now(rp, d.A.rp, st_);
     ords.push_back(bank_order(rp));
     tail_ = l;
   }
@@ -877,7 +891,7 @@ void DevHier::build_tail() {
   std::vector<int*> ord_dev(cnt);
   for (int k = 0; k < cnt; ++k) {
     ord_dev[k] = alloc<int>(ords[k].size());
-    DR_CK(cudaMemcpy(ord_dev[k], ords[k].data(), ords[k].size() * sizeof(int), cudaMemcpyHostToDevice));
+    h2d(ord_dev[k], ords[k], st_);
   }
   auto make = [&](auto tag) {
     using T = decltype(tag);
@@ -974,11 +988,11 @@ void DevHier::build_tail() {
     cl.bytes = 0;
     for (const TailCopy& c : pat) cl.bytes += c.bytes;
     TailCopy* dl = alloc<TailCopy>(pat.size());
-    DR_CK(cudaMemcpy(dl, pat.data(), pat.size() * sizeof(TailCopy), cudaMemcpyHostToDevice));
+    h2d(dl, pat, st_);
     cl.list = dl;
     allow_tail_smem<T>();
     TailLevel<T>* dst = alloc<TailLevel<T>>(cnt);
-    DR_CK(cudaMemcpy(dst, v.data(), cnt * sizeof(TailLevel<T>), cudaMemcpyHostToDevice));
+    h2d_now(dst, v, st_);
     return (void*)dst;
   };
   tail64_ = make(double());
@@ -1017,7 +1031,7 @@ void DevHier::build_fused(const HostHierarchy& H) {
     }
     if (!ok) continue;
     d.pq_pos = alloc<int>(pos.size());
-    DR_CK(cudaMemcpy(d.pq_pos, pos.data(), pos.size() * sizeof(int), cudaMemcpyHostToDevice));
+    h2d_now(d.pq_pos, pos, st_);
     d.q = alloc<double>(d.AP.nnz + 4);
     spgemm<double>(d.AP, d.A, d.P, d.AP.v, d.A.v, d.P.v, nullptr);
     d.fuse_up = true;
@@ -1464,8 +1478,8 @@ void DevHier::build_transpose() {
   for (auto& d : L_) {
     const int n = d.A.n;
     std::vector<int> rp(n + 1), ci(d.A.nnz);
-    DR_CK(cudaMemcpy(rp.data(), d.A.rp, rp.size() * sizeof(int), cudaMemcpyDeviceToHost));
-    if (!ci.empty()) DR_CK(cudaMemcpy(ci.data(), d.A.ci, ci.size() * sizeof(int), cudaMemcpyDeviceToHost));
+    d2h_now(rp, d.A.rp, st_);
+    d2h_now(ci, d.A.ci, st_);
     std::vector<int> trp(n + 1, 0), tci(ci.size()), perm(ci.size());
     for (int k = 0; k < (int)ci.size(); ++k) ++trp[ci[k] + 1];
     for (int j = 0; j < n; ++j) trp[j + 1] += trp[j];

@@ -75,6 +75,26 @@ def test_cycles_around_resetups(make):
     assert not np.array_equal(want_a, want_b)
 
 
+def test_host_values_of_a_resetup_arrive():
+    """The level values on the device are the ones given, on every one of many
+    fresh hierarchies (the upload must be ordered before its use)."""
+    A, cfg = gauss_seidel_2d()
+    B = A.copy()
+    B.data = B.data * np.random.default_rng(1).uniform(0.9, 1.1, B.nnz)
+    x, b = vectors(A.shape[0])
+    first = None
+    for _ in range(30):
+        h = draugr.amg_setup(A, cfg)
+        before = cycle(h, cfg, x, b)
+        cycle(h, cfg, x, b)
+        draugr.amg_resetup(h, B, cfg)
+        assert np.array_equal(h.export(0, "A_nzval"), B.data)
+        got = (before, cycle(h, cfg, x, b))
+        first = first or got
+        assert np.array_equal(got[0], first[0]) and np.array_equal(got[1], first[1])
+        h.free()
+
+
 def test_more_options_than_graphs():
     A, cfg = gauss_seidel_2d()
     x, b = vectors(A.shape[0])
