@@ -93,3 +93,52 @@ def test_cycle_through_the_coarsest_inverse(coarse):
     x = draugr.amg_cycle(np.zeros(A.shape[0]), b, h, cfg)
     ref = oracle.OracleHierarchy(h).cycle(np.zeros(A.shape[0]), b)
     assert np.linalg.norm(x - ref) < 1e-12 * np.linalg.norm(ref)
+
+
+def neumann(m, shift):
+    """Heterogeneous diffusion on m^3 cells without a boundary condition,
+    plus `shift` on the diagonal: nearly singular on every level."""
+    kap = np.exp(1.5 * np.random.default_rng(3).standard_normal(m ** 3))
+    idx = np.arange(m ** 3).reshape(m, m, m)
+    r, c, v = [], [], []
+    for ax in range(3):
+        a, b = np.take(idx, range(m - 1), ax).ravel(), np.take(idx, range(1, m), ax).ravel()
+        w = 2 / (1 / kap[a] + 1 / kap[b])
+        r += [a, b]
+        c += [b, a]
+        v += [-w, -w]
+    A = sp.csr_matrix((np.concatenate(v), (np.concatenate(r), np.concatenate(c))), shape=(m ** 3, m ** 3))
+    return sp.csr_matrix(A + sp.diags(shift - np.asarray(A.sum(1)).ravel())).sorted_indices()
+
+
+def pcg(A, M, b, tol, maxiter):
+    x, r, p, rz = np.zeros_like(b), b.copy(), None, 0.0
+    for it in range(1, maxiter + 1):
+        z = M(r)
+        rz, old = r @ z, rz
+        p = z if p is None else z + rz / old * p
+        q = A @ p
+        alpha = rz / (p @ q)
+        x, r = x + alpha * p, r - alpha * q
+        if np.linalg.norm(r) < tol * np.linalg.norm(b):
+            break
+    return x, it
+
+
+@pytest.mark.parametrize("shift", [1e-3, 1e-6, 1e-9])
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+def test_nearly_singular_coarsest_system(shift, precision):
+    """The explicit inverse where it could lose most: a coarsest system of
+    33 to 64 unknowns with a condition of up to 1e11.  PCG takes as many
+    iterations as with the oracle's substitutions, to the same residual."""
+    A = neumann(32, shift)
+    cfg = draugr.hypre_default_config(agg_trunc_factor=0.2, smoother=draugr.L1JacobiSmootherType(), seed=3,
+                                      max_coarse_size=64)
+    h = draugr.amg_setup(A, cfg)
+    assert 33 <= int(h.level_info(-1)[0]) <= 64
+    O = oracle.OracleHierarchy(h)
+    b = A @ np.random.default_rng(1).uniform(-1, 1, A.shape[0])
+    want, steps = pcg(A, lambda r: O.cycle(np.zeros_like(r), r), b, 1e-8, 200)
+    x, it, _ = draugr.pcg(np.zeros_like(b), b, h, cfg, tol=1e-8, maxiter=200, precision=precision)
+    assert abs(it - steps) <= 1
+    assert np.linalg.norm(b - A @ x) < max(1.01e-8 * np.linalg.norm(b), 1.5 * np.linalg.norm(b - A @ want))

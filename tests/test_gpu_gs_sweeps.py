@@ -60,22 +60,30 @@ def sweeps(A, order, off, invd, x, b, steps):
     return x
 
 
+# matrix, and whether each precision's sweeps are one cluster launch
 CASES = {
-    "rows_700_short": lambda: long_rows(3000, 3, 700),          # 8 lanes per row, remainder loop
-    "rows_900_long": lambda: long_rows(400, 40, 390),           # 32 lanes per row
-    "poisson1d_5": lambda: problems.poisson1d(5),
-    "poisson2d_46": lambda: problems.poisson2d(46, 44),         # 2 colours of 1012 rows: the cluster
-    "poisson2d_47": lambda: problems.poisson2d(47, 46),         # of 1081: a launch per colour
-    "fe27_15": lambda: problems.anisotropic_27pt(15),           # 8 colours of about 420 rows: a launch per colour
-    "banded_27000": lambda: banded(27000, 115),                 # 116 colours: FP64 iterate just fits
-    "banded_29100": lambda: banded(29100, 115),                 # it does not
+    "rows_700_short": (lambda: long_rows(3000, 3, 700), True, True),       # 8 lanes per row, remainder loop
+    "rows_900_long": (lambda: long_rows(400, 40, 390), True, True),        # 32 lanes per row
+    "poisson1d_5": (lambda: problems.poisson1d(5), True, True),
+    "poisson2d_46": (lambda: problems.poisson2d(46, 44), True, True),      # 2 colours of 1012 rows
+    "poisson2d_47": (lambda: problems.poisson2d(47, 46), False, False),    # of 1081: a launch per colour
+    "fe27_15": (lambda: problems.anisotropic_27pt(15), True, True),        # 8 colours of about 420 rows
+    "banded_27000": (lambda: banded(27000, 115), True, True),              # 116 colours: FP64 iterate just fits
+    "banded_29100": (lambda: banded(29100, 115), False, True),             # it does not
 }
+
+
+def launched(lib, h, x, b, steps, prec):
+    before = lib.draugr_b200_kernel_launches()
+    got = h.level_op(0, 2, x, b, steps=steps, precision=prec)
+    return got, lib.draugr_b200_kernel_launches() - before
 
 
 @pytest.mark.parametrize("smoother", [draugr.ColoredGaussSeidelType, draugr.L1ColoredGaussSeidelType])
 @pytest.mark.parametrize("name", list(CASES))
 def test_gs_sweeps(name, smoother):
-    A = CASES[name]()
+    make, *cluster = CASES[name]
+    A = make()
     n = A.shape[0]
     h = draugr.amg_setup(A, draugr.AMGConfig(coarsening=draugr.AggregationCoarsening(0.25), smoother=smoother(),
                                              max_coarse_size=2, max_levels=3))
@@ -83,13 +91,17 @@ def test_gs_sweeps(name, smoother):
     rng = np.random.default_rng(1)
     x, b = rng.uniform(-1, 1, n), rng.uniform(-1, 1, n)
     longest = int(np.diff(A.indptr).max())
-    for steps in (1, 2, 3):
-        ref = sweeps(A, order, off, invd, x, b, steps)
-        for prec, eps in ((0, 2.2e-16), (1, 1.2e-7)):
-            got = h.level_op(0, 2, x, b, steps=steps, precision=prec)
+    lib = draugr.load()
+    for prec, eps in ((0, 2.2e-16), (1, 1.2e-7)):
+        h.level_op(0, 2, x, b, steps=1, precision=prec)  # the first FP32 call also converts the matrix
+        count = {}
+        for steps in (1, 2, 3):
+            ref = sweeps(A, order, off, invd, x, b, steps)
+            got, count[steps] = launched(lib, h, x, b, steps, prec)
             # a row's sum of `longest` products in another order, every sweep
             tol = 4 * eps * longest * steps
             assert np.linalg.norm(got - ref) <= tol * np.linalg.norm(ref), (steps, prec)
+        assert count[3] - count[1] == (0 if cluster[prec] else 2 * (len(off) - 1))
 
 
 # one launch per colour: matrix, lanes per row of its kernel
@@ -127,14 +139,12 @@ def test_colour_launches(name):
     x, b = rng.uniform(-1, 1, n), rng.uniform(-1, 1, n)
     lib = draugr.load()
     for prec, eps in ((0, 2.2e-16), (1, 1.2e-7)):
-        count = []
+        h.level_op(0, 2, x, b, steps=1, precision=prec)
+        count = {}
         for steps in (1, 3):
             ref = sweeps(A, order, off, invd, x, b, steps)
-            before = lib.draugr_b200_kernel_launches()
-            got = h.level_op(0, 2, x, b, steps=steps, precision=prec)
-            count.append(lib.draugr_b200_kernel_launches() - before)
+            got, count[steps] = launched(lib, h, x, b, steps, prec)
             # a row's sum of `longest` products in another order, every sweep
             assert np.linalg.norm(got - ref) <= 4 * eps * longest * steps * np.linalg.norm(ref), (steps, prec)
-        if prec == 0:  # FP32's first call also converts the matrix
-            assert count[1] - count[0] == 2 * (len(off) - 1)
+        assert count[3] - count[1] == 2 * (len(off) - 1)
     h.free()

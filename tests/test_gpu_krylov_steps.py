@@ -1,7 +1,7 @@
 """BiCGStab and FGMRES with their scalars on the device: iterates after a few
-steps against NumPy with the oracle's cycle as the preconditioner (a step
-enqueued past the last one must not change x), and the transposed coarsest
-solve at the edges of its kernels."""
+steps against NumPy with the oracle's cycle as the preconditioner, solves that
+stop by their tolerance with the next step already enqueued (which must not
+change x), and the transposed coarsest solve at the edges of its kernels."""
 
 import numpy as np
 import pytest
@@ -22,9 +22,12 @@ def system(m=24, coarse=30):
 
 
 def bicgstab(A, M, b, steps):
+    """Per step: the iterate after its half step and after it, and the
+    relative norms of s and r."""
     x, r = np.zeros_like(b), b.copy()
     rh, p, v = r.copy(), np.zeros_like(b), np.zeros_like(b)
     rho = alpha = omega = 1.0
+    out, bn = [], np.linalg.norm(b)
     for _ in range(steps):
         rho1 = rh @ r
         p = r + (rho1 / rho) * (alpha / omega) * (p - omega * v)
@@ -35,23 +38,49 @@ def bicgstab(A, M, b, steps):
         sh = M(s)
         t = A @ sh
         omega = (t @ s) / (t @ t)
-        x = x + alpha * ph + omega * sh
+        half = x + alpha * ph
+        x = half + omega * sh
         r = s - omega * t
         rho = rho1
-    return x
+        out.append((half, x, np.linalg.norm(s) / bn, np.linalg.norm(r) / bn))
+    return out
 
 
 @pytest.mark.parametrize("steps", [1, 2, 3, 5])
 def test_bicgstab_iterates(steps):
     A, cfg, h, b = system()
     O = oracle.OracleHierarchy(h)
-    ref = bicgstab(A, lambda r: O.cycle(np.zeros_like(r), r), b, steps)
+    ref = bicgstab(A, lambda r: O.cycle(np.zeros_like(r), r), b, steps)[-1][1]
     for _ in range(3):  # launched directly, captured, replayed
         x, it, rel = draugr.bicgstab(np.zeros_like(b), b, h, cfg, tol=1e-14, maxiter=steps)
         assert it == steps
         # rounding grows with the steps' condition; 1e-12 per step measured
         assert np.linalg.norm(x - ref) < 1e-10 * np.linalg.norm(ref)
         assert abs(rel - np.linalg.norm(b - A @ x) / np.linalg.norm(b)) < 1e-12
+
+
+@pytest.mark.parametrize("half", [False, True], ids=["full_step", "half_step"])
+def test_bicgstab_stops_with_a_step_enqueued(half):
+    """A tolerance that step k meets first, at its end or at its half: the
+    step enqueued behind it leaves x alone."""
+    A, cfg, h, b = system()
+    O = oracle.OracleHierarchy(h)
+    steps = bicgstab(A, lambda r: O.cycle(np.zeros_like(r), r), b, 9)
+    norms = [v for st in steps for v in st[2:]]  # in the order the tests see them
+    pick = [i for i in range(2 if half else 3, len(norms), 2) if norms[i] < 0.6 * min(norms[:i])]
+    assert pick
+    for i in pick:
+        k, tol = i // 2 + 1, 1.2 * norms[i]
+        want = steps[k - 1][0 if half else 1]
+        for _ in range(3):  # launched directly, captured, replayed
+            x, it, rel = draugr.bicgstab(np.zeros_like(b), b, h, cfg, tol=tol, maxiter=50)
+            assert it == k
+            # rounding grows with the steps' condition; 1e-12 per step measured
+            assert np.linalg.norm(x - want) < 1e-10 * np.linalg.norm(want)
+            assert abs(rel - norms[i]) < 1e-8 * norms[i] + 1e-12
+        if not half:  # the same solve with no step behind it
+            y, it, _ = draugr.bicgstab(np.zeros_like(b), b, h, cfg, tol=tol, maxiter=k)
+            assert it == k and np.array_equal(x, y)
 
 
 @pytest.mark.parametrize("precision", ["fp64", "mixed"])
