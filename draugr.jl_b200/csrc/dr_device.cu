@@ -147,9 +147,11 @@ std::vector<int> make_tiles(const std::vector<int>& rp, const std::vector<int>& 
 static_assert(kTileCap == kRowTileCap, "host and device tile capacities differ");
 
 // Launch with programmatic stream serialization: the kernel may begin
-// while the previous kernel in the stream drains.  Only for kernels that
-// read nothing but sparsity patterns before pdl_wait() (k_tile_rows,
-// k_coarse_tail, k_pcg_update).
+// while the previous kernel in the stream drains.  Only for kernels that read
+// before pdl_wait() nothing but what no kernel in flight writes: patterns,
+// and matrix values and factors, whose writers (setup, ensure_fp32,
+// build_transpose, resetup) end with a stream synchronisation.  With
+// cluster > 1 the grid is made of clusters of that many blocks.
 template <typename... KArgs, typename... Args>
 void launch_cluster(int cluster, void (*kern)(KArgs...), int grid, int block, size_t smem, cudaStream_t st,
                     Args&&... args) {
@@ -1743,7 +1745,8 @@ int DevHier::fgmres(double* x, const double* b, const CycleOpts& o, double tol, 
     counted();
     // about one wave of blocks over all columns (352 blocks of 256 rows for
     // each of 30 columns took 12 us at 90 k rows, 5.8 us this way)
-    k_mdot<<<dim3(std::max(1, std::min(gx, max_grid_ / k)), k), kBlock, 0, st_>>>(n, V, (long long)n, vw, gm_part_, gm_tk_, h);
+    const int blocks = std::max(1, std::min(gx, max_grid_ / k));
+    k_mdot<<<dim3(blocks, k), kBlock, 0, st_>>>(n, V, (long long)n, vw, gm_part_, gm_tk_, h);
   };
   auto maxpy = [&](int k, const double* Mv, const double* h, double sign, double* out) {
     counted();

@@ -9,7 +9,8 @@
 // is the chain from colour to colour.  Measured on the default configuration
 // at 64^3 (458 colours on 7 levels, FP64 PCG, 14 iterations): 82.7 ms with
 // plain launches, 40.4 ms with dependent launches that load a row's entries
-// ahead, 16.0 ms with the cluster kernel on the levels it fits.  Two kernels:
+// ahead, 16.0 ms with the cluster kernel on the levels it fits (14.9 ms with the
+// later changes to the other kernels of the cycle).  Two kernels:
 //
 //   k_gs_cluster  every colour of every sweep in one launch of one
 //       thread-block cluster.  Each block keeps the whole iterate in its

@@ -2236,16 +2236,16 @@ k_spgemm_warp(int nrows, const int* __restrict__ out_rp, const int* __restrict__
 // b into x, in the operation order of k_lu_solve (so each system's coarse
 // solve gives what its own hierarchy's gives).
 // The explicit inverses of the coarsest systems of a batch (block k: system
-// k; inverse stored where the factors are;
-// n <= kInvMax),
-// and their application x = A^-1 b, one block of kInvMax threads per
-// system, each row of the inverse summed in column order.  Latency-bound: the
-// right-hand side sits in shared memory and 16 entries of the inverse are in
-// flight (64 systems, 16 batched PCG iterations: 25.8 ms with both read one
-// after the other, 25.4 ms so).
-__global__ void __launch_bounds__(kInvThreads) k_lu_inverse_batch(const int* __restrict__ nb, const long long* __restrict__ luoff,
-                                   const int* __restrict__ poff, const double* __restrict__ lu_all,
-                                   const int* __restrict__ piv_all, double* __restrict__ inv_all) {
+// k; inverse stored where the factors are; n <= kInvMax), and their
+// application x = A^-1 b, one block of kInvMax threads per system, each row of
+// the inverse summed in column order.  Latency-bound: the right-hand side sits
+// in shared memory and 16 entries of the inverse are in flight (64 systems, 16
+// batched PCG iterations: 25.8 ms with both read one after the other, 25.4 ms
+// so).
+__global__ void __launch_bounds__(kInvThreads)
+k_lu_inverse_batch(const int* __restrict__ nb, const long long* __restrict__ luoff, const int* __restrict__ poff,
+                   const double* __restrict__ lu_all, const int* __restrict__ piv_all,
+                   double* __restrict__ inv_all) {
   const int k = blockIdx.x;
   lu_inverse_block(nb[k], lu_all + luoff[k], piv_all + poff[k], inv_all + luoff[k]);
 }
