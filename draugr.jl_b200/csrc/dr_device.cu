@@ -1123,9 +1123,11 @@ static_assert(kern::kGsBatch == 8, "gs_color_lanes counts on 8 entries per lane"
 // holds, on average, no more rows than the cluster has row groups (one round
 // each; 256 groups of 32 lanes, 1024 of 8); else one launch per colour.  With
 // two rounds a colour the cluster's 16 SMs cannot stream the rows as fast as
-// the whole GPU: level 2 of the 64^3 heterogeneous problem (57 colours of 490
-// rows) takes 173 us per sweep in the cluster and 125 us in 57 launches,
-// level 3 (108 colours of 94 rows) 93 against 280 us.
+// the whole GPU.  us per FP64 sweep in the cluster and in launches, by rows per
+// colour (entries per row): 8 lanes, 512 (5) 1.9, 6.2; 691 (18) 14, 23; 1012 (5)
+// 4.4, 6.2; 1250 (9) 11, 7.4; 1639 (18) 36, 22; 2048 (5) 7.5, 3.2; 32 lanes, 21
+// (57) 12, 59; 93 (205) 81, 293; 385 (26) 26, 30; 490 (125) 173, 125; 1000 (24)
+// 37, 15.
 template <typename T>
 void DevHier::gs_sweeps(const DevLevel& L, const DevMat& A, const T* b, T* x, int steps) {
   if (steps <= 0 || A.n <= 0) return;
