@@ -355,7 +355,9 @@ class Hierarchy:
 
     def set_stream(self, stream) -> None:
         """Run on a CUDA stream: a torch.cuda.Stream, a raw cudaStream_t
-        (int) or None for the library's own stream."""
+        (int) or None for the library's own stream.  Calls with device arrays
+        read them on that stream: on another stream than the one that writes
+        them, synchronise first (amg_solve_diff and nz_gradient do)."""
         raw = getattr(stream, "cuda_stream", stream)
         _lib.check(_lib.load().draugr_b200_set_stream(self.handle, raw), "set_stream")
 
@@ -535,9 +537,19 @@ def nz_gradient(h: Hierarchy, x, lam):
     lib = _lib.load()
     nnz = int(h.level_info(0)[1]) if h.nlevels > 0 else int(h.level_info(-1)[1])
     grad = torch.empty(nnz, dtype=torch.float64, device=x.device)
+    _finish_torch_work(grad)
     _lib.check(lib.draugr_b200_nz_gradient_device(h.handle, x.numel(), x.data_ptr(), lam.data_ptr(),
                                                   grad.data_ptr()), "nz_gradient")
     return grad
+
+
+def _finish_torch_work(t):
+    """Wait for what torch has enqueued on the current stream (among it the
+    operands and the memory of `t`): the hierarchy runs on a stream of its
+    own unless set_stream says otherwise."""
+    import torch
+
+    torch.cuda.current_stream(t.device).synchronize()
 
 
 class _Solve:
@@ -564,9 +576,11 @@ def amg_solve_diff(values, b, h: Hierarchy, config: AMGConfig | None = None, tol
         class Fn(torch.autograd.Function):
             @staticmethod
             def forward(ctx, values, b, h, config, tol, maxiter, symmetric, precision):
-                amg_resetup(h, values.detach().contiguous(), config)
+                vv = values.detach().contiguous()
                 x = torch.zeros_like(b)
                 bb = b.detach().contiguous()
+                _finish_torch_work(x)
+                amg_resetup(h, vv, config)
                 if symmetric:
                     _, it, rel = pcg(x, bb, h, config, tol=tol, maxiter=maxiter, precision=precision)
                 else:
@@ -581,6 +595,7 @@ def amg_solve_diff(values, b, h: Hierarchy, config: AMGConfig | None = None, tol
                 (x,) = ctx.saved_tensors
                 lam = torch.zeros_like(x)
                 g = gx.contiguous()
+                _finish_torch_work(lam)
                 if ctx.symmetric:
                     pcg(lam, g, ctx.h, ctx.config, tol=ctx.tol, maxiter=ctx.maxiter, precision=ctx.precision)
                 else:

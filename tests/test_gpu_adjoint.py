@@ -206,3 +206,39 @@ def test_fp32_cycle_gradient(name):
         check_finite_differences(h, make, kappa, b, S, d, symmetric, L, gk, rng, tol=1e-15, rtol=1e-4)
     else:
         check_finite_differences(h, make, kappa, b, S, d, symmetric, L, gk, rng, precision="mixed")
+
+
+@pytest.mark.parametrize("symmetric", [False, True])
+def test_gradient_of_operands_still_being_computed(symmetric):
+    """Values, right-hand side and the loss's gradient at the end of a queue
+    of torch work that is not waited for (the hierarchy runs on a stream of
+    its own): the same gradients as with finished operands."""
+    A = problems.poisson2d(48)
+    n = A.shape[0]
+    h = draugr.amg_setup(A, CFG)
+    rng = np.random.default_rng(3)
+    host = torch.tensor(rng.uniform(0.95, 1.05, A.nnz) * A.data) if not symmetric else torch.tensor(A.data * 1.25)
+    b0, w0 = torch.tensor(rng.uniform(-1, 1, n)).cuda(), torch.tensor(rng.uniform(-1, 1, n)).cuda()
+    v0, big = host.cuda(), torch.randn(4096, 4096, device="cuda")
+
+    def busy():  # about 50 ms of matrix products whose result is zero
+        y = big
+        for _ in range(20):
+            y = torch.clamp(y @ big, -1.0, 1.0)
+        return (y[0, 0] * 0.0).double()
+
+    def grads(wait):
+        zero = busy()
+        vals, b = (v0 + zero).requires_grad_(), (b0 + zero).requires_grad_()
+        if wait:
+            torch.cuda.synchronize()
+        x = draugr.amg_solve_diff(vals, b, h, CFG, tol=1e-12, symmetric=symmetric)
+        w = w0 + busy()
+        if wait:
+            torch.cuda.synchronize()
+        return torch.autograd.grad((x * w).sum(), (vals, b))
+
+    want = grads(True)
+    for _ in range(3):
+        for g, ref in zip(grads(False), want):
+            assert torch.equal(g, ref)
